@@ -14,7 +14,8 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libncs_b200.so")
-SOURCES = ["ncs_capi.cu", "ncs_plain.cu", "ncs_warp.cu", "ncs_spectral.cu", "ncs_noalloc.cu",
+SOURCES = ["ncs_capi.cu", "ncs_plain.cu", "ncs_warp.cu", "ncs_spectral.cu", "ncs_pair.cu",
+           "ncs_noalloc.cu",
            "ncs_net.cu", "ncs_masks.cu", "ncs_sim.cu",
            "ncs_norm.cu", "ncs_net_tc.cu", "ncs_adu.cu", "ncs_tc.cu"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]

@@ -19,6 +19,9 @@ cudaError_t launch_warp_blocks(const SolveArgs& args, int grid, int blocks, cuda
 int warp_max_ctas_per_sm(int m, int blocks);
 cudaError_t launch_spectral(const SolveArgs& args, int grid, int blocks, cudaStream_t stream);
 int spectral_max_ctas_per_sm(int m, int blocks, bool warm, bool batch);
+cudaError_t launch_pair(const SolveArgs& args, int ctas_per_sm, int num_sms, cudaStream_t stream);
+cudaError_t pair_prepare(bool warm, bool batch);
+bool pair_one_wave(long long n_tiles, int ctas_per_sm, int num_sms);
 cudaError_t launch_tc(const SolveArgs& args, bool bf16x3, int grid, cudaStream_t stream);
 int tc_max_ctas_per_sm(bool bf16x3, bool warm);
 int tc_tiles_per_cta();
@@ -200,7 +203,12 @@ void lane_layout(const float nat[256], float* out) {
 // queue: the work counter of this launch (default: the handle's own)
 int launch(ncsb_handle* h, ncsb::SolveArgs& a, cudaStream_t s, unsigned long long* queue = nullptr) {
     if (!queue) queue = h->d_queue;
-    cudaError_t e = cudaMemsetAsync(queue, 0, sizeof(unsigned long long), s);
+    // the default form at m = 1 runs two tiles per warp (ncs_pair.cu); a launch
+    // that gives each pair its own warp leaves the work counter alone
+    const bool pair = h->p.mode == NCSB_MODE_SPECTRAL && h->p.m <= 1;
+    cudaError_t e = cudaSuccess;
+    if (!pair || !ncsb::pair_one_wave(a.n_tiles, h->p.ctas_per_sm, h->num_sms))
+        e = cudaMemsetAsync(queue, 0, sizeof(unsigned long long), s);
     if (e != cudaSuccess) return cuda_fail(h, e, "cudaMemsetAsync(queue)");
     a.queue = queue;
     a.msq = h->d_msq;
@@ -210,6 +218,11 @@ int launch(ncsb_handle* h, ncsb::SolveArgs& a, cudaStream_t s, unsigned long lon
     a.min_step = (float)h->p.min_step;
     a.max_iters = h->p.max_iters;
     a.m = h->p.m;
+    if (pair) {
+        e = ncsb::launch_pair(a, h->p.ctas_per_sm, h->num_sms, s);
+        if (e != cudaSuccess) return cuda_fail(h, e, "kernel launch");
+        return NCSB_OK;
+    }
     const bool wg = h->p.mode == NCSB_MODE_PLAIN_WG;
     const bool spec = h->p.mode == NCSB_MODE_SPECTRAL;
     if (h->p.mode == NCSB_MODE_TC_TF32 || h->p.mode == NCSB_MODE_TC_BF16X3) {
@@ -766,8 +779,11 @@ int ncsb_batch_set(ncsb_handle* h, const ncsb_stack* stacks, int n_stacks) {
     h->n_stacks = n_stacks;
     h->batch_tiles = total;
     // resolve the kernel variants' attributes now, outside any stream capture
-    ncsb::spectral_max_ctas_per_sm(h->p.m, 0, false, true);
-    ncsb::spectral_max_ctas_per_sm(h->p.m, 0, true, true);
+    for (const bool warm : {false, true}) {
+        ncsb::spectral_max_ctas_per_sm(h->p.m, 0, warm, true);
+        e = ncsb::pair_prepare(warm, true);
+        if (e != cudaSuccess) return cuda_fail(h, e, "kernel attributes");
+    }
     return NCSB_OK;
 }
 

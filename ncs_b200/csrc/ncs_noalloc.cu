@@ -31,6 +31,7 @@ cudaError_t launch_warp_blocks(const SolveArgs& args, int grid, int blocks, cuda
 int warp_max_ctas_per_sm(int m, int blocks);
 cudaError_t launch_spectral(const SolveArgs& args, int grid, int blocks, cudaStream_t stream);
 int spectral_max_ctas_per_sm(int m, int blocks, bool warm, bool batch);
+cudaError_t launch_pair(const SolveArgs& args, int ctas_per_sm, int num_sms, cudaStream_t stream);
 }  // namespace ncsb
 
 using ncsb::tiles_along;
@@ -166,6 +167,9 @@ extern "C" int ncsb_reduce_noise_noalloc(const ncsb_params* p, const float* mask
     a.min_step = (float)p->min_step;
     a.max_iters = p->max_iters;
     a.m = p->m;
+    if (p->mode == NCSB_MODE_SPECTRAL && p->m <= 1)
+        return ncsb::launch_pair(a, p->ctas_per_sm, dev->num_sms, s) == cudaSuccess ? NCSB_OK
+                                                                                   : NCSB_ECUDA;
     const bool wg = p->mode == NCSB_MODE_PLAIN_WG;
     const bool spec = p->mode == NCSB_MODE_SPECTRAL;
     const int per_sm = p->ctas_per_sm > 0

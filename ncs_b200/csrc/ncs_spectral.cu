@@ -1,5 +1,6 @@
 // ncs_spectral.cu -- L-BFGS with a spectral initial inverse Hessian, one warp
-// per 16x16 tile (NCSB_MODE_SPECTRAL, the default form).
+// per 16x16 tile (NCSB_MODE_SPECTRAL with history sizes above 1; at m = 1, the
+// default, ncs_pair.cu runs the same algorithm two tiles per warp).
 //
 // The per-tile cost (clib/pyCNCS/ncs.c:185-299, cuda/ncs.cu:635-817) has the
 // Hessian
@@ -49,11 +50,9 @@ __host__ __device__ constexpr size_t spec_warp_bytes(int m, bool vg) {
            (3 * (size_t)m + (vg ? 4 : 2)) * 32 * 2 * sizeof(float4);
 }
 
-// The 5-CTA launch of the plain single-stack solve keeps v = 2 alpha Q u and
-// g in the warp's shared memory instead of registers: at the 96 registers that
-// 5 CTAs (20 warps) per SM allow, the solve then runs without spills and
-// 0.7 % faster than 4 CTAs with them in registers; at 4 CTAs the extra loads
-// measured 0.6 % slower.
+// A 5-CTA launch (ctas_per_sm >= 5) of a plain single-stack solve keeps v =
+// 2 alpha Q u and g in the warp's shared memory instead of registers: the 96
+// registers that 5 CTAs (20 warps) per SM allow do not hold them.
 template <int MinBlocks, bool Warm, bool Batch>
 __host__ __device__ constexpr bool vg_shared() {
     return MinBlocks >= 5 && !Warm && !Batch;
@@ -671,24 +670,18 @@ KernelFn spectral_variant_m(int blocks, bool warm, bool batch) {
 }
 
 KernelFn spectral_variant(int blocks, int m, bool warm, bool batch) {
-    return m <= 1 ? spectral_variant_m<1>(blocks, warm, batch)
-                  : (m <= 2 ? spectral_variant_m<2>(blocks, warm, batch)
-                            : spectral_variant_m<4>(blocks, warm, batch));
+    return m <= 2 ? spectral_variant_m<2>(blocks, warm, batch)
+                  : spectral_variant_m<4>(blocks, warm, batch);
 }
 
-int spectral_default_blocks(int m, bool warm, bool batch) {
+int spectral_default_blocks(int m) {
     int dev = 0, per_sm = 0;
     cudaGetDevice(&dev);
     if (cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev) !=
         cudaSuccess)
         per_sm = 228 * 1024;
-    // Plain single-stack solves at m = 1: 5 CTAs (20 warps, 96 registers, v and
-    // g in shared memory) measured fastest.  Otherwise 4 CTAs (16 warps, 128
-    // registers): with more history, proposals or a batch the 5-CTA budget
-    // spills.
-    if (m <= 1 && !warm && !batch &&
-        (int)(per_sm / (spectral_smem_bytes(m, true) + 1024)) >= 5)
-        return 5;
+    // at most 4 CTAs (16 warps, 128 registers): the 5-CTA budget spills with
+    // two or more history pairs
     const int b = (int)(per_sm / (spectral_smem_bytes(m, false) + 1024));
     return b < 4 ? b : 4;
 }
@@ -697,7 +690,7 @@ int spectral_default_blocks(int m, bool warm, bool batch) {
 
 cudaError_t launch_spectral(const SolveArgs& args, int grid, int blocks, cudaStream_t stream) {
     const bool warm = args.u0 != nullptr, batch = args.stacks != nullptr;
-    const int b = blocks > 0 ? blocks : spectral_default_blocks(args.m, warm, batch);
+    const int b = blocks > 0 ? blocks : spectral_default_blocks(args.m);
     const size_t smem = spectral_smem_bytes(args.m, variant_vg(b, warm, batch));
     const KernelFn fn = spectral_variant(b, args.m, warm, batch);
     cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -707,7 +700,7 @@ cudaError_t launch_spectral(const SolveArgs& args, int grid, int blocks, cudaStr
 }
 
 int spectral_max_ctas_per_sm(int m, int blocks, bool warm, bool batch) {
-    const int b = blocks > 0 ? blocks : spectral_default_blocks(m, warm, batch);
+    const int b = blocks > 0 ? blocks : spectral_default_blocks(m);
     const size_t smem = spectral_smem_bytes(m, variant_vg(b, warm, batch));
     const KernelFn fn = spectral_variant(b, m, warm, batch);
     if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
