@@ -21,6 +21,7 @@
 
 #include "../../include/ncs_b200.h"
 #include "ncs_internal.cuh"
+#include "ncs_wino.cuh"
 
 namespace ncsb {
 namespace net {
@@ -230,8 +231,9 @@ __global__ void adam_step(float* __restrict__ w, const float* __restrict__ g, fl
     w[i] -= lr * (mi / bc1) / (sqrtf(vi / bc2) + eps);
 }
 
-// Tile mean and (std + 1) of one value per thread of a 256-thread CTA.
-__device__ __forceinline__ float2 tile_scale(float dv, float* red) {
+// Tile mean and (std + 1) of one value per thread of 8 warps: each warp's sums
+// into red[16], then (after a barrier) the statistics from them.
+__device__ __forceinline__ void tile_sums(float dv, float* red) {
     float s1 = dv, s2 = dv * dv;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -242,7 +244,8 @@ __device__ __forceinline__ float2 tile_scale(float dv, float* red) {
         red[threadIdx.x >> 5] = s1;
         red[8 + (threadIdx.x >> 5)] = s2;
     }
-    __syncthreads();
+}
+__device__ __forceinline__ float2 tile_stats(const float* red) {
     float a = 0.0f, q = 0.0f;
 #pragma unroll
     for (int w = 0; w < 8; ++w) {
@@ -262,7 +265,9 @@ __global__ void __launch_bounds__(256) features(const float* __restrict__ d,
     const int t = blockIdx.x;
     if (t >= n) return;
     const float dv = d[(size_t)t * 256 + threadIdx.x], gv = gam[(size_t)t * 256 + threadIdx.x];
-    const float2 ms = tile_scale(dv, red);
+    tile_sums(dv, red);
+    __syncthreads();
+    const float2 ms = tile_stats(red);
     x[(size_t)t * 512 + threadIdx.x] = (dv - ms.x) / ms.y;
     x[(size_t)t * 512 + 256 + threadIdx.x] = sqrtf(fmaxf(dv, 0.0f) + fmaxf(gv, 0.0f)) / ms.y;
     if (threadIdx.x == 0) {
@@ -272,19 +277,6 @@ __global__ void __launch_bounds__(256) features(const float* __restrict__ d,
 }
 
 // ---- fused inference -------------------------------------------------------
-
-// One conv layer from planes xin to planes yout (interior), shared memory only.
-template <int CIN, int COUT, bool RELU>
-__device__ __forceinline__ void layer_smem(const float* xin, float* yout, const float* wt,
-                                           const float* b, int r, int c) {
-    float acc[COUT];
-#pragma unroll
-    for (int co = 0; co < COUT; ++co) acc[co] = b[co];
-    conv_pixel<CIN, COUT>(xin, wt, r, c, acc);
-#pragma unroll
-    for (int co = 0; co < COUT; ++co)
-        yout[co * kCS + (r + 1) * kPad + c + 1] = RELU ? fmaxf(acc[co], 0.0f) : acc[co];
-}
 
 struct InferSrc {
     int tile_mode;
@@ -297,97 +289,175 @@ struct InferSrc {
     int n_stacks;
 };
 
-constexpr size_t infer_smem_bytes() {
-    return ((size_t)round4(kParams) + 2 * (size_t)round4(kC * kCS)) * sizeof(float);
-}
+// Shared memory of the fused inference, in floats: both hidden layers'
+// transformed weights, the activation planes, the Winograd exchange buffer, then
+// the first and last layer's weights, the biases, the input planes and the sums
+// of the tile scale.  The last layer's weights are [ci][12] (9 taps).
+struct InferSmem {
+    static constexpr int u2 = 0, u3 = u2 + wino::kU, planes = u3 + wino::kU,
+                         vm = planes + wino::kPlanes, w1 = vm + wino::kV(16), b1 = w1 + 2 * 9 * kC,
+                         b2 = b1 + kC, b3 = b2 + kC, w4 = b3 + kC, b4 = w4 + 12 * kC,
+                         xin = b4 + 4, red = xin + 2 * wino::kPlane, end = red + 16;
+};
+constexpr size_t kInferSmem = InferSmem::end * sizeof(float);
+constexpr int kInferThreads = 256;
 
-// Persistent grid; one tile per CTA at a time, activations ping-pong between
-// two 32-channel plane sets, weights resident in shared memory.
-__global__ void __launch_bounds__(256) infer(const InferSrc src, const float* __restrict__ params,
-                                             float* __restrict__ u0) {
+// Persistent grid, one CTA (8 warps) per SM and one tile per CTA at a time:
+// first layer direct, the 32 -> 32 layers by Winograd's F(2x2, 3x3) in place
+// (ncs_wino.cuh), last layer direct over strips of four pixels.  The direct form
+// of all layers took one float4 weight broadcast per 4 multiply-adds and was
+// bound by the shared-memory pipe (96 % busy): 20 x 512^2 frames 9.15 ms, this 3.72
+// ms (FMA pipe 51 %, shared memory 79 % of the time); error against FP64 3.1e-7
+// direct, 1.4e-7 this.
+__global__ void __launch_bounds__(kInferThreads) infer(const InferSrc src,
+                                                        const float* __restrict__ params,
+                                                        float* __restrict__ u0) {
+    using S = InferSmem;
+    constexpr int kRow = wino::kRow, kPlane = wino::kPlane;
     extern __shared__ __align__(16) float sm[];
-    float* wsm = sm;
-    float* a0 = sm + round4(kParams);
-    float* a1 = a0 + round4(kC * kCS);
-    __shared__ float red[16];
-    for (int i = threadIdx.x; i < kParams; i += blockDim.x) wsm[i] = params[i];
-    for (int i = threadIdx.x; i < 2 * round4(kC * kCS); i += blockDim.x) a0[i] = 0.0f;
-    __syncthreads();
-    const float* w1 = wsm;
-    const float* b1 = w1 + 2 * 9 * kC;
-    const float* w2 = b1 + kC;
-    const float* b2 = w2 + kC * 9 * kC;
-    const float* w3 = b2 + kC;
-    const float* b3 = w3 + kC * 9 * kC;
-    const float* w4 = b3 + kC;
-    const float* b4 = w4 + kC * 9;
-    const int p = threadIdx.x, r = p >> 4, c = p & 15;
+    float* planes = sm + S::planes;
+    float* xin = sm + S::xin;
+    const int t = threadIdx.x, lane = t & 31;
+    constexpr int o2 = 2 * 9 * kC + kC, o3 = o2 + kC * 9 * kC + kC, o4 = o3 + kC * 9 * kC + kC;
+    wino::weights(sm + S::u2, params + o2, false);
+    wino::weights(sm + S::u3, params + o3, false);
+    for (int i = t; i < 2 * 9 * kC + kC; i += kInferThreads) sm[S::w1 + i] = params[i];
+    for (int i = t; i < 9 * kC; i += kInferThreads) sm[S::w4 + (i / 9) * 12 + i % 9] = params[o4 + i];
+    if (t == 0) sm[S::b4] = params[o4 + 9 * kC];
+    for (int i = t; i < wino::kPlanes; i += kInferThreads) planes[i] = 0.0f;
+    for (int i = t; i < 2 * kPlane; i += kInferThreads) xin[i] = 0.0f;
+    const float bias2 = params[o3 - kC + lane], bias3 = params[o4 - kC + lane];
+    // a thread's pixel: a warp holds rows r and r + 2, on distinct banks
+    const int r = ((t >> 6) << 2) + ((t >> 5) & 1) + 2 * ((t >> 4) & 1), c = t & 15;
     const long long per_frame = (long long)src.tiles_x * src.tiles_y;
-    for (long long tile = blockIdx.x; tile < src.n_tiles; tile += gridDim.x) {
-        float dv, gv;
+    auto pixel = [&](long long tile, float& dv, float& gv) {
         if (src.tile_mode) {
-            dv = src.d[tile * 256 + p];
-            gv = src.gamma[tile * 256 + p];
-        } else {
-            const float* sd = src.d;
-            const float* sgam = src.gamma;
-            long long gstride = src.gamma_frame_stride, lt = tile, pf = per_frame;
-            int H = src.H, W = src.W, ty = src.tiles_y;
-            if (src.stacks) {  // batched: the last stack whose first tile is <= tile
-                int lo = 0, hi = src.n_stacks - 1;
-                while (lo < hi) {
-                    const int mid = (lo + hi + 1) >> 1;
-                    if (src.stacks[mid].tile_begin <= tile) lo = mid;
-                    else hi = mid - 1;
-                }
-                const StackDesc& st = src.stacks[lo];
-                sd = st.data;
-                sgam = st.gamma;
-                gstride = st.gamma_frame_stride;
-                lt = tile - st.tile_begin;
-                H = st.H;
-                W = st.W;
-                ty = st.tiles_y;
-                pf = (long long)st.tiles_x * st.tiles_y;
-            }
-            const int f = (int)(lt / pf);
-            const int rem = (int)(lt - (long long)f * pf);
-            const int ti = rem / ty, tj = rem - ti * ty;
-            const int yy = clampi(tile_origin(ti, H) + r - 1, 0, H - 1);
-            const int xx = clampi(tile_origin(tj, W) + c - 1, 0, W - 1);
-            dv = sd[(long long)f * H * W + (long long)yy * W + xx];
-            gv = sgam[(long long)f * gstride + (long long)yy * W + xx];
+            dv = src.d[tile * 256 + r * 16 + c];
+            gv = src.gamma[tile * 256 + r * 16 + c];
+            return;
         }
-        __syncthreads();  // the previous tile is done with red[] and the planes
-        const float2 ms = tile_scale(dv, red);
-        a1[(r + 1) * kPad + c + 1] = (dv - ms.x) / ms.y;
-        a1[kCS + (r + 1) * kPad + c + 1] = sqrtf(fmaxf(dv, 0.0f) + fmaxf(gv, 0.0f)) / ms.y;
+        const float* sd = src.d;
+        const float* sgam = src.gamma;
+        long long gstride = src.gamma_frame_stride, lt = tile, pf = per_frame;
+        int H = src.H, W = src.W, ty = src.tiles_y;
+        if (src.stacks) {  // batched: the last stack whose first tile is <= tile
+            int lo = 0, hi = src.n_stacks - 1;
+            while (lo < hi) {
+                const int mid = (lo + hi + 1) >> 1;
+                if (src.stacks[mid].tile_begin <= tile) lo = mid;
+                else hi = mid - 1;
+            }
+            const StackDesc& st = src.stacks[lo];
+            sd = st.data;
+            sgam = st.gamma;
+            gstride = st.gamma_frame_stride;
+            lt = tile - st.tile_begin;
+            H = st.H;
+            W = st.W;
+            ty = st.tiles_y;
+            pf = (long long)st.tiles_x * st.tiles_y;
+        }
+        const int f = (int)(lt / pf);
+        const int rem = (int)(lt - (long long)f * pf);
+        const int ti = rem / ty, tj = rem - ti * ty;
+        const int yy = clampi(tile_origin(ti, H) + r - 1, 0, H - 1);
+        const int xx = clampi(tile_origin(tj, W) + c - 1, 0, W - 1);
+        dv = sd[(long long)f * H * W + (long long)yy * W + xx];
+        gv = sgam[(long long)f * gstride + (long long)yy * W + xx];
+    };
+    float dn = 0.0f, gn = 0.0f;
+    if (blockIdx.x < src.n_tiles) pixel(blockIdx.x, dn, gn);
+    for (long long tile = blockIdx.x; tile < src.n_tiles; tile += gridDim.x) {
+        const float dv = dn, gv = gn;
+        if (tile + gridDim.x < src.n_tiles) pixel(tile + gridDim.x, dn, gn);
+        // tile mean and std + 1, then the two feature planes
+        tile_sums(dv, sm + S::red);
         __syncthreads();
-        layer_smem<2, kC, true>(a1, a0, w1, b1, r, c);
+        const float2 ms = tile_stats(sm + S::red);
+        xin[(r + 1) * kRow + c + 1] = (dv - ms.x) / ms.y;
+        xin[kPlane + (r + 1) * kRow + c + 1] = sqrtf(fmaxf(dv, 0.0f) + fmaxf(gv, 0.0f)) / ms.y;
         __syncthreads();
-        layer_smem<kC, kC, true>(a0, a1, w2, b2, r, c);
+        {  // layer 1: thread = pixel, all output channels
+            float2 acc[16];
+#pragma unroll
+            for (int q = 0; q < 16; ++q)
+                acc[q] = *reinterpret_cast<const float2*>(sm + S::b1 + 2 * q);
+#pragma unroll
+            for (int ci = 0; ci < 2; ++ci)
+#pragma unroll
+                for (int k = 0; k < 9; ++k) {
+                    const float2 x2 = warp::splat(xin[ci * kPlane + (r + k / 3) * kRow + c + k % 3]);
+                    const float4* wr = reinterpret_cast<const float4*>(sm + S::w1 + (ci * 9 + k) * kC);
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) {
+                        const float4 w = wr[q];
+                        acc[2 * q] = warp::fma2(make_float2(w.x, w.y), x2, acc[2 * q]);
+                        acc[2 * q + 1] = warp::fma2(make_float2(w.z, w.w), x2, acc[2 * q + 1]);
+                    }
+                }
+            float* o = planes + (r + 1) * kRow + c + 1;
+#pragma unroll
+            for (int q = 0; q < 16; ++q) {
+                o[2 * q * kPlane] = fmaxf(acc[q].x, 0.0f);
+                o[(2 * q + 1) * kPlane] = fmaxf(acc[q].y, 0.0f);
+            }
+        }
         __syncthreads();
-        layer_smem<kC, kC, true>(a1, a0, w3, b3, r, c);
+#pragma unroll 1
+        for (int l = 0; l < 2; ++l) {
+            float out[32];
+            wino::layer<16>(planes, sm + (l ? S::u3 : S::u2), sm + S::vm, l ? bias3 : bias2, out);
+#pragma unroll
+            for (int k = 0; k < 32; ++k) out[k] = fmaxf(out[k], 0.0f);
+            wino::store_planes<16>(planes, out);
+            __syncthreads();
+        }
+        {  // layer 4: thread = strip of 4 pixels x 8 input channels
+            const int sr = (t & 63) >> 2, sc = 4 * (t & 3), g = t >> 6;
+            float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll 4
+            for (int i = 0; i < 8; ++i) {
+                const float* x = planes + (8 * g + i) * kPlane + sr * kRow + sc;
+                const float4* w4 = reinterpret_cast<const float4*>(sm + S::w4 + (8 * g + i) * 12);
+                const float4 wa = w4[0], wb = w4[1], wc = w4[2];
+                const float w[9] = {wa.x, wa.y, wa.z, wa.w, wb.x, wb.y, wb.z, wb.w, wc.x};
+#pragma unroll
+                for (int ky = 0; ky < 3; ++ky) {
+                    float v[6];
+#pragma unroll
+                    for (int k = 0; k < 3; ++k) {
+                        const float2 z = *reinterpret_cast<const float2*>(x + ky * kRow + 2 * k);
+                        v[2 * k] = z.x;
+                        v[2 * k + 1] = z.y;
+                    }
+#pragma unroll
+                    for (int kx = 0; kx < 3; ++kx)
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) acc[e] = fmaf(w[3 * ky + kx], v[e + kx], acc[e]);
+                }
+            }
+            *reinterpret_cast<float4*>(sm + S::vm + g * 256 + sr * 16 + sc) =
+                make_float4(acc[0], acc[1], acc[2], acc[3]);
+        }
         __syncthreads();
-        float y[1] = {b4[0]};
-        conv_pixel<kC, 1>(a0, w4, r, c, y);
+        const float* part = sm + S::vm + r * 16 + c;
+        float y = sm[S::b4];
+#pragma unroll
+        for (int g = 0; g < 4; ++g) y += part[g * 256];
         const float lo = kStartFrac * fmaxf(dv + gv, 1e-3f) - gv;
-        u0[tile * 256 + p] = fmaxf(fmaf(ms.y, y[0], dv), lo);
+        u0[tile * 256 + r * 16 + c] = fmaxf(fmaf(ms.y, y, dv), lo);
     }
 }
 
 int launch_infer(const InferSrc& src, const float* params, float* u0, cudaStream_t s) {
-    const size_t smem = infer_smem_bytes();
-    if (cudaFuncSetAttribute(infer, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-        cudaSuccess)
+    if (cudaFuncSetAttribute(infer, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)kInferSmem) != cudaSuccess)
         return NCSB_ECUDA;
-    int dev = 0, sms = 1, per_sm = 1;
+    int dev = 0, sms = 1;
     if (cudaGetDevice(&dev) != cudaSuccess) return NCSB_ECUDA;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, infer, 256, smem);
-    long long grid = (long long)sms * (per_sm > 0 ? per_sm : 1);
-    if (grid > src.n_tiles) grid = src.n_tiles;
-    infer<<<(unsigned)grid, 256, smem, s>>>(src, params, u0);
+    const long long grid = src.n_tiles < sms ? src.n_tiles : sms;
+    infer<<<(unsigned)grid, kInferThreads, kInferSmem, s>>>(src, params, u0);
     return cudaGetLastError() == cudaSuccess ? NCSB_OK : NCSB_ECUDA;
 }
 
