@@ -402,6 +402,26 @@ int ncsb_net_conv_fwd(const float *x, const float *wt, const float *b, float *y,
 int ncsb_net_conv_wgrad(const float *x, const float *dy, float *dwt, float *db, int n_tiles,
                         int cin, int cout, void *stream);
 
+/* Backward passes of a training step of n tiles.  Every [n][32][16][16] array is
+ * 16-byte aligned; gradients and the loss are added to.
+ * ncsb_net_conv_xgrad: input gradient dx of a 32 -> 32 layer with weights
+ * wt [32][9][32] from its output gradient dy, zero where act <= 0 (act: the
+ * layer's input, a ReLU's output; NULL: no mask).
+ * ncsb_net_last_layer: from a [n][32][16][16] (the last layer's input, a ReLU's
+ * output) and target [n][16][16], the loss sum (y - target)^2 / (256 n), the
+ * gradients dwt [32][9] and db [1], and g [n][32][16][16], the gradient with
+ * respect to that ReLU's input.
+ * ncsb_net_first_layers_grad: the first layer's gradients dwt [2][9][32] and
+ * db [32] from dy [n][32][16][16], the output gradient of the second layer
+ * (weights wt [32][9][32]), act [n][32][16][16], its input, and x
+ * [n][2][16][16], the first layer's input. */
+int ncsb_net_conv_xgrad(const float *dy, const float *wt, const float *act, float *dx, int n_tiles,
+                        void *stream);
+int ncsb_net_last_layer(const float *a, const float *wt, const float *b, const float *target,
+                        float *g, float *dwt, float *db, float *loss, int n_tiles, void *stream);
+int ncsb_net_first_layers_grad(const float *dy, const float *wt, const float *act, const float *x,
+                               float *dwt, float *db, int n_tiles, void *stream);
+
 /* Weights of the input-gradient convolution: wf[cout][8 - tap][cin] =
  * wt[cin][tap][cout], so that ncsb_net_conv_fwd(dy, wf, NULL, dx, n, cout,
  * cin, 0) gives dx = conv3x3^T(dy). */

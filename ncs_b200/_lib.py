@@ -117,6 +117,7 @@ EXPORTS = [
     "ncsb_set_otf_mask", "ncsb_num_tiles", "ncsb_reduce_noise", "ncsb_solve_tiles",
     "ncsb_reduce_noise_noalloc", "ncsb_reduce_noise_start",
     "ncsb_net_param_count", "ncsb_net_conv_fwd", "ncsb_net_conv_wgrad", "ncsb_net_flip",
+    "ncsb_net_conv_xgrad", "ncsb_net_last_layer", "ncsb_net_first_layers_grad",
     "ncsb_net_relu_bwd", "ncsb_net_mse_grad", "ncsb_net_adam", "ncsb_net_features",
     "ncsb_net_infer_stack", "ncsb_net_infer_tiles", "ncsb_net_infer_batch",
     "ncsb_batch_set", "ncsb_batch_num_tiles", "ncsb_batch_reduce_noise",
@@ -178,6 +179,11 @@ def load():
     lib.ncsb_net_conv_fwd.argtypes = [vp, vp, vp, vp, ci, ci, ci, ci, vp]
     lib.ncsb_net_conv_wgrad.argtypes = [vp, vp, vp, vp, ci, ci, ci, vp]
     lib.ncsb_net_flip.argtypes = [vp, vp, ci, ci, vp]
+    lib.ncsb_net_conv_xgrad.argtypes = [vp, vp, vp, vp, ci, vp]
+    lib.ncsb_net_last_layer.argtypes = [vp] * 8 + [ci, vp]
+    lib.ncsb_net_first_layers_grad.argtypes = [vp] * 6 + [ci, vp]
+    for name in ("ncsb_net_conv_xgrad", "ncsb_net_last_layer", "ncsb_net_first_layers_grad"):
+        getattr(lib, name).restype = ctypes.c_int
     lib.ncsb_net_relu_bwd.argtypes = [vp, vp, i64, vp]
     lib.ncsb_net_mse_grad.argtypes = [vp, vp, vp, vp, i64, vp]
     lib.ncsb_net_adam.argtypes = [vp, vp, vp, vp, i64, f32, f32, f32, f32, ci, vp]

@@ -488,6 +488,51 @@ int launch_wgrad(const float* x, const float* dy, float* dwt, float* db, int n, 
     return cudaGetLastError() == cudaSuccess ? NCSB_OK : NCSB_ECUDA;
 }
 
+// The Winograd kernels of the 32 -> 32 layers read and write 16 bytes at a time.
+bool aligned16(const void* a, const void* b, const void* c) {
+    return (((uintptr_t)a | (uintptr_t)b | (uintptr_t)c) & 15) == 0;
+}
+
+int one_per_sm(int n) {
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return n < sms ? n : sms;
+}
+
+template <bool RELU, bool FLIP, bool FIRST>
+int launch_wino(const float* x, const float* wt, const float* b, const float* act, float* y, int n,
+                cudaStream_t s, const float* f = nullptr, float* dw = nullptr,
+                float* db = nullptr) {
+    const auto kernel = wino::conv<RELU, FLIP, FIRST>;
+    const size_t smem = FIRST ? wino::kFirstSmem : wino::kConvSmem;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
+        cudaSuccess)
+        return NCSB_ECUDA;
+    kernel<<<one_per_sm(n), wino::kThreads, smem, s>>>(x, wt, b, act, y, n, f, dw, db);
+    return cudaGetLastError() == cudaSuccess ? NCSB_OK : NCSB_ECUDA;
+}
+
+int launch_wino_wgrad(const float* x, const float* dy, float* dwt, float* db, int n,
+                      cudaStream_t s) {
+    if (cudaFuncSetAttribute(wino::wgrad, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)wino::kWgradSmem) != cudaSuccess)
+        return NCSB_ECUDA;
+    wino::wgrad<<<one_per_sm(n), wino::kThreads, wino::kWgradSmem, s>>>(x, dy, dwt, db, n);
+    return cudaGetLastError() == cudaSuccess ? NCSB_OK : NCSB_ECUDA;
+}
+
+int launch_last(const float* a, const float* wt, const float* b, const float* target, float* g,
+                float* dwt, float* db, float* loss, int n, cudaStream_t s) {
+    if (cudaFuncSetAttribute(wino::last_layer, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)wino::kLastSmem) != cudaSuccess)
+        return NCSB_ECUDA;
+    const int grid = 2 * one_per_sm((n + 1) / 2);  // two CTAs per SM
+    wino::last_layer<<<grid < n ? grid : n, wino::kThreads, wino::kLastSmem, s>>>(
+        a, wt, b, target, g, dwt, db, loss, n);
+    return cudaGetLastError() == cudaSuccess ? NCSB_OK : NCSB_ECUDA;
+}
+
 int launch_infer_batch(const float* params, const StackDesc* stacks, int n_stacks,
                        long long n_tiles, float* u0, cudaStream_t s) {
     if (n_tiles == 0) return NCSB_OK;
@@ -518,6 +563,9 @@ int ncsb_net_conv_fwd(const float* x, const float* wt, const float* b, float* y,
     cudaStream_t s = (cudaStream_t)stream;
     if (cin == 2 && cout == 32)
         return relu ? launch_fwd<2, 32, true>(x, wt, b, y, n, s) : launch_fwd<2, 32, false>(x, wt, b, y, n, s);
+    if (cin == 32 && cout == 32 && aligned16(x, y, y))
+        return relu ? launch_wino<true, false, false>(x, wt, b, nullptr, y, n, s)
+                    : launch_wino<false, false, false>(x, wt, b, nullptr, y, n, s);
     if (cin == 32 && cout == 32)
         return relu ? launch_fwd<32, 32, true>(x, wt, b, y, n, s) : launch_fwd<32, 32, false>(x, wt, b, y, n, s);
     if (cin == 32 && cout == 1)
@@ -533,9 +581,34 @@ int ncsb_net_conv_wgrad(const float* x, const float* dy, float* dwt, float* db, 
     if (n == 0) return NCSB_OK;
     cudaStream_t s = (cudaStream_t)stream;
     if (cin == 2 && cout == 32) return launch_wgrad<2, 32>(x, dy, dwt, db, n, s);
+    if (cin == 32 && cout == 32 && aligned16(x, dy, dy)) return launch_wino_wgrad(x, dy, dwt, db, n, s);
     if (cin == 32 && cout == 32) return launch_wgrad<32, 32>(x, dy, dwt, db, n, s);
     if (cin == 32 && cout == 1) return launch_wgrad<32, 1>(x, dy, dwt, db, n, s);
     return NCSB_EINVAL;
+}
+
+int ncsb_net_conv_xgrad(const float* dy, const float* wt, const float* act, float* dx, int n,
+                        void* stream) {
+    if (!dy || !wt || !dx || n < 0 || !aligned16(dy, act, dx)) return NCSB_EINVAL;
+    if (n == 0) return NCSB_OK;
+    return launch_wino<false, true, false>(dy, wt, nullptr, act, dx, n, (cudaStream_t)stream);
+}
+
+int ncsb_net_first_layers_grad(const float* dy, const float* wt, const float* act, const float* x,
+                               float* dwt, float* db, int n, void* stream) {
+    if (!dy || !wt || !act || !x || !dwt || !db || n < 0 || !aligned16(dy, act, act))
+        return NCSB_EINVAL;
+    if (n == 0) return NCSB_OK;
+    return launch_wino<false, true, true>(dy, wt, nullptr, act, nullptr, n, (cudaStream_t)stream, x,
+                                          dwt, db);
+}
+
+int ncsb_net_last_layer(const float* a, const float* wt, const float* b, const float* target,
+                        float* g, float* dwt, float* db, float* loss, int n, void* stream) {
+    if (!a || !wt || !b || !target || !g || !dwt || !db || !loss || n < 0 || !aligned16(a, g, g))
+        return NCSB_EINVAL;
+    if (n == 0) return NCSB_OK;
+    return launch_last(a, wt, b, target, g, dwt, db, loss, n, (cudaStream_t)stream);
 }
 
 int ncsb_net_flip(const float* wt, float* wf, int cin, int cout, void* stream) {

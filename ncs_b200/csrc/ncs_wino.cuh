@@ -41,7 +41,7 @@ constexpr int kPlane = 434;
 constexpr int kPlanes = kC * kPlane;
 // U[point][ci][co], V[point][ci][patch] and M[point][patch][co] (in V's place)
 constexpr int kU = 16 * kC * kC;
-constexpr int kV(int cp) { return 16 * kC * cp; }
+__host__ __device__ constexpr int kV(int cp) { return 16 * kC * cp; }
 
 // U = G g G' of wt[ci][tap][co] (flip: of the input gradient's filter, whose
 // channels are exchanged and whose taps are reversed), in FP64, rounded once.
@@ -178,6 +178,427 @@ __device__ __forceinline__ void store_planes(float* planes, const float (&out)[5
         float* p = planes + lane * kPlane + (2 * (pos >> 3) + 1) * kRow + 2 * (pos & 7) + 1;
 #pragma unroll
         for (int e = 0; e < 4; ++e) p[(e >> 1) * kRow + (e & 1)] = out[4 * q + e];
+    }
+}
+
+// Of the convolution kernels (a layer at a time): CP = 32, 16 warps
+constexpr int kCp = 32, kThreads = 16 * kCp;
+
+// The thread's 16 values of a [kC][16][16] tile, as four float4s: channel and
+// row of each from load_at().
+__device__ __forceinline__ int tile_at(int q) { return q * kThreads + threadIdx.x; }  // float4 index
+__device__ __forceinline__ void load_tile(const float* __restrict__ x, float4 (&v)[4]) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) v[q] = __ldg(reinterpret_cast<const float4*>(x) + tile_at(q));
+}
+__device__ __forceinline__ void tile_to_planes(const float4 (&v)[4], float* planes) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const int i = tile_at(q), ch = i >> 6, r = (i >> 2) & 15, c4 = 4 * (i & 3);
+        float* p = planes + ch * kPlane + (r + 1) * kRow + c4 + 1;
+        p[0] = v[q].x;
+        p[1] = v[q].y;
+        p[2] = v[q].z;
+        p[3] = v[q].w;
+    }
+}
+
+// The kernels of a training step.  2048 tiles take 0.14 ms a layer here and 0.13
+// ms in wgrad (direct kernels: 0.56 and 0.46 ms); a step 2.91 -> 0.94 ms, its
+// gradient's error against FP64 6.5e-7 -> 3.7e-7.
+//
+// y = conv(x, wt) + b per tile (b may be null), then ReLU (RELU), or the gradient
+// mask of a ReLU whose output is act (act non-null: y = 0 where act <= 0).  FLIP:
+// the convolution is the input gradient's, with wt the forward weights.  FIRST:
+// y is the output gradient of the first layer, whose two input channels are f:
+// it is not stored but reduced to that layer's weight gradient in dw [2][9][32]
+// and db (128 MB less traffic per step of 2048 tiles than a pass of its own).
+template <bool RELU, bool FLIP, bool FIRST>
+__global__ void __launch_bounds__(kThreads) conv(const float* __restrict__ x,
+                                                 const float* __restrict__ wt,
+                                                 const float* __restrict__ b,
+                                                 const float* __restrict__ act,
+                                                 float* __restrict__ y, int n,
+                                                 const float* __restrict__ f,
+                                                 float* __restrict__ dw, float* __restrict__ db) {
+    extern __shared__ __align__(16) float sm[];
+    float* U = sm;
+    float* planes = U + kU;
+    float* vm = planes + kPlanes;
+    float* fp = vm + kV(kCp);  // FIRST: the feature planes, 18 rows of kRow, 2 channels
+    const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+    for (int i = t; i < kPlanes; i += kThreads) planes[i] = 0.0f;
+    if (FIRST)
+        for (int i = t; i < 2 * kPlane; i += kThreads) fp[i] = 0.0f;
+    weights(U, wt, FLIP);
+    const float bias = b ? b[lane] : 0.0f;
+    float tot[FIRST ? 19 : 1] = {};  // FIRST: this lane's channel: 18 weights and the bias
+    float4 next[4];
+    int tile = blockIdx.x;
+    if (tile < n) load_tile(x + (size_t)tile * kC * 256, next);
+    for (; tile < n; tile += gridDim.x) {
+        __syncthreads();  // weights and borders written; the last tile's planes read
+        tile_to_planes(next, planes);
+        if (FIRST)
+            fp[(t >> 8) * kPlane + (((t >> 4) & 15) + 1) * kRow + (t & 15) + 1] =
+                __ldg(f + (size_t)tile * 512 + t);
+        if (tile + gridDim.x < n) load_tile(x + (size_t)(tile + gridDim.x) * kC * 256, next);
+        __syncthreads();
+        float out[16];
+        layer<kCp>(planes, U, vm, bias, out);
+        if (RELU) {
+#pragma unroll
+            for (int k = 0; k < 16; ++k) out[k] = fmaxf(out[k], 0.0f);
+        }
+        store_planes<kCp>(planes, out);
+        __syncthreads();
+        float4* yt = FIRST ? nullptr : reinterpret_cast<float4*>(y + (size_t)tile * kC * 256);
+        const float4* at =
+            act ? reinterpret_cast<const float4*>(act + (size_t)tile * kC * 256) : nullptr;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int i = tile_at(q), ch = i >> 6, r = (i >> 2) & 15, c4 = 4 * (i & 3);
+            float* p = planes + ch * kPlane + (r + 1) * kRow + c4 + 1;
+            float4 o = make_float4(p[0], p[1], p[2], p[3]);
+            if (act) {
+                const float4 a = __ldg(at + i);
+                o.x = a.x > 0.0f ? o.x : 0.0f;
+                o.y = a.y > 0.0f ? o.y : 0.0f;
+                o.z = a.z > 0.0f ? o.z : 0.0f;
+                o.w = a.w > 0.0f ? o.w : 0.0f;
+            }
+            if (FIRST) {
+                p[0] = o.x;
+                p[1] = o.y;
+                p[2] = o.z;
+                p[3] = o.w;
+            } else {
+                yt[i] = o;
+            }
+        }
+        if (FIRST) {  // lane = output channel, warp = row
+            __syncthreads();
+            float g[16], acc[18];
+            const float* p = planes + lane * kPlane + (w + 1) * kRow + 1;
+#pragma unroll
+            for (int c = 0; c < 16; ++c) {
+                g[c] = p[c];
+                tot[18] += g[c];
+            }
+#pragma unroll
+            for (int k = 0; k < 18; ++k) acc[k] = 0.0f;
+#pragma unroll
+            for (int k = 0; k < 6; ++k) {  // input channel and window row
+                const float* xr = fp + (k / 3) * kPlane + (w + k % 3) * kRow;
+                float v[20];
+#pragma unroll
+                for (int q = 0; q < 5; ++q) {
+                    const float2 a = *reinterpret_cast<const float2*>(xr + 4 * q);
+                    const float2 c = *reinterpret_cast<const float2*>(xr + 4 * q + 2);
+                    v[4 * q] = a.x;
+                    v[4 * q + 1] = a.y;
+                    v[4 * q + 2] = c.x;
+                    v[4 * q + 3] = c.y;
+                }
+#pragma unroll
+                for (int kx = 0; kx < 3; ++kx)
+#pragma unroll
+                    for (int c = 0; c < 16; ++c)
+                        acc[3 * k + kx] = fmaf(g[c], v[c + kx], acc[3 * k + kx]);
+            }
+#pragma unroll
+            for (int k = 0; k < 18; ++k) tot[k] += acc[k];
+        }
+    }
+    if (FIRST) {
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < 19; ++k) vm[(w * 19 + k) * kC + lane] = tot[k];
+        __syncthreads();
+        for (int i = t; i < 19 * kC; i += kThreads) {
+            double s = 0.0;
+            for (int k = 0; k < 16; ++k) s += vm[k * 19 * kC + i];
+            atomicAdd(i < 18 * kC ? dw + i : db + (i - 18 * kC), (float)s);
+        }
+    }
+}
+
+constexpr size_t kConvSmem = (size_t)(kU + kPlanes + kV(kCp)) * sizeof(float);
+constexpr size_t kFirstSmem = kConvSmem + 2 * kPlane * sizeof(float);
+
+// Weight gradient: dL/dg = G' [ sum (A dy A') . (B' d B) ] G, db = sum dy.  Warp
+// w accumulates point w's 32 x 32 products over all patches of the CTA's tiles
+// in registers; one atomic per weight and CTA at the end.
+constexpr int kG = 258;  // dy plane stride: 64-bit reads over channels hit distinct banks
+constexpr int kP = 512;  // V and dY: [point][patch][channel]
+constexpr size_t kWgradSmem =
+    (size_t)(kPlanes + kC * kG + 2 * 16 * kP) * sizeof(float);
+
+__global__ void __launch_bounds__(kThreads) wgrad(const float* __restrict__ x,
+                                                  const float* __restrict__ dy,
+                                                  float* __restrict__ dwt, float* __restrict__ db,
+                                                  int n) {
+    extern __shared__ __align__(16) float sm[];
+    float* planes = sm;
+    float* gs = planes + kPlanes;
+    float* V = gs + kC * kG;
+    float* Y = V + 16 * kP;
+    const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+    for (int i = t; i < kPlanes; i += kThreads) planes[i] = 0.0f;
+    const int ig = lane >> 3, og = lane & 7;  // 8 input and 4 output channels
+    float2 acc[8][2];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) acc[i][0] = acc[i][1] = make_float2(0.0f, 0.0f);
+    double bsum = 0.0;
+    float4 nx[4], ng[4];
+    int tile = blockIdx.x;
+    if (tile < n) {
+        load_tile(x + (size_t)tile * kC * 256, nx);
+        load_tile(dy + (size_t)tile * kC * 256, ng);
+    }
+    for (; tile < n; tile += gridDim.x) {
+        __syncthreads();  // the last tile's planes are read, the borders written
+        tile_to_planes(nx, planes);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int i = tile_at(q);
+            float* p = gs + (i >> 6) * kG + 4 * (i & 63);
+            *reinterpret_cast<float2*>(p) = make_float2(ng[q].x, ng[q].y);
+            *reinterpret_cast<float2*>(p + 2) = make_float2(ng[q].z, ng[q].w);
+        }
+        if (tile + gridDim.x < n) {
+            load_tile(x + (size_t)(tile + gridDim.x) * kC * 256, nx);
+            load_tile(dy + (size_t)(tile + gridDim.x) * kC * 256, ng);
+        }
+        __syncthreads();
+#pragma unroll 1
+        for (int c = 0; c < 4; ++c) {
+            const int tr = 2 * c + (w >> 3), tj = w & 7;  // this warp's patch
+            {
+                float v[16];
+                patch_in(planes + lane * kPlane + 2 * tr * kRow + 2 * tj, v);
+#pragma unroll
+                for (int k = 0; k < 16; ++k) V[k * kP + t] = v[k];
+            }
+            {
+                const float* p = gs + lane * kG + 32 * tr + 2 * tj;
+                const float2 a = *reinterpret_cast<const float2*>(p);
+                const float2 b = *reinterpret_cast<const float2*>(p + 16);
+                bsum += (double)((a.x + a.y) + (b.x + b.y));
+                const float2 rows[4] = {a, make_float2(a.x + b.x, a.y + b.y),
+                                        make_float2(a.x - b.x, a.y - b.y), make_float2(-b.x, -b.y)};
+#pragma unroll
+                for (int y = 0; y < 4; ++y) {
+                    Y[(4 * y + 0) * kP + t] = rows[y].x;
+                    Y[(4 * y + 1) * kP + t] = rows[y].x + rows[y].y;
+                    Y[(4 * y + 2) * kP + t] = rows[y].x - rows[y].y;
+                    Y[(4 * y + 3) * kP + t] = -rows[y].y;
+                }
+            }
+            __syncthreads();
+            const float* vp = V + w * kP + 8 * ig;
+            const float* yp = Y + w * kP + 4 * og;
+#pragma unroll 4
+            for (int k = 0; k < 16; ++k) {
+                const float4 v0 = *reinterpret_cast<const float4*>(vp + k * kC);
+                const float4 v1 = *reinterpret_cast<const float4*>(vp + k * kC + 4);
+                const float4 g = *reinterpret_cast<const float4*>(yp + k * kC);
+                const float2 g0 = make_float2(g.x, g.y), g1 = make_float2(g.z, g.w);
+                const float vi[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    acc[i][0] = fma2(splat(vi[i]), g0, acc[i][0]);
+                    acc[i][1] = fma2(splat(vi[i]), g1, acc[i][1]);
+                }
+            }
+            __syncthreads();
+        }
+    }
+    // M[point][ci][co] through shared memory (V and dY's 16 x 1024 floats)
+    float* M = V;
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+        *reinterpret_cast<float4*>(M + w * 1024 + (8 * ig + i) * kC + 4 * og) =
+            make_float4(acc[i][0].x, acc[i][0].y, acc[i][1].x, acc[i][1].y);
+    reinterpret_cast<double*>(gs)[t] = bsum;  // [warp][channel]
+    __syncthreads();
+    for (int idx = t; idx < kC * kC; idx += kThreads) {
+        const int ci = idx >> 5, co = idx & 31;
+        float m[4][4], r[3][4];
+#pragma unroll
+        for (int k = 0; k < 16; ++k) m[k >> 2][k & 3] = M[k * 1024 + idx];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            const float p = 0.5f * (m[1][c] + m[2][c]), q = 0.5f * (m[1][c] - m[2][c]);
+            r[0][c] = m[0][c] + p;
+            r[1][c] = q;
+            r[2][c] = p + m[3][c];
+        }
+#pragma unroll
+        for (int y = 0; y < 3; ++y) {
+            const float p = 0.5f * (r[y][1] + r[y][2]), q = 0.5f * (r[y][1] - r[y][2]);
+            float* o = dwt + (ci * 9 + 3 * y) * kC + co;
+            atomicAdd(o, r[y][0] + p);
+            atomicAdd(o + kC, q);
+            atomicAdd(o + 2 * kC, p + r[y][3]);
+        }
+    }
+    if (t < kC) {
+        double s = 0.0;
+        for (int k = 0; k < 16; ++k) s += reinterpret_cast<const double*>(gs)[k * kC + t];
+        atomicAdd(db + t, (float)s);
+    }
+}
+
+// The last layer (32 -> 1) of a training step in one pass over its input: output,
+// MSE loss against target, weight and bias gradients, and the input gradient g
+// masked by the ReLU that made a.  Separate kernels read a three times and ran
+// 74 + 7 + 271 + 30 us for 2048 tiles.  Sums over tiles are FP64.
+constexpr int kLastPart = 8 * 256;
+constexpr size_t kLastSmem = (size_t)(kPlanes + kLastPart + kPlane + 2 + 12 * kC + 64) * sizeof(float);
+
+__global__ void __launch_bounds__(kThreads, 2) last_layer(
+    const float* __restrict__ a, const float* __restrict__ wt, const float* __restrict__ b,
+    const float* __restrict__ target, float* __restrict__ g, float* __restrict__ dwt,
+    float* __restrict__ db, float* __restrict__ loss, int n) {
+    extern __shared__ __align__(16) float sm[];
+    float* planes = sm;
+    float* part = planes + kPlanes;
+    float* gp = part + kLastPart;  // dL/dy, zero-bordered
+    float* ws = gp + kPlane + 2;   // [ci][12], 16-byte aligned
+    double* red = reinterpret_cast<double*>(ws + 12 * kC);
+    const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+    for (int i = t; i < kPlanes; i += kThreads) planes[i] = 0.0f;
+    for (int i = t; i < kPlane; i += kThreads) gp[i] = 0.0f;
+    for (int i = t; i < 9 * kC; i += kThreads) ws[(i / 9) * 12 + i % 9] = wt[i];
+    const float bias = b[0];
+    const double inv = 1.0 / ((double)n * 256.0);
+    const int sr = (t & 63) >> 2, sc = 4 * (t & 3), grp = t >> 6;  // strip, 4 channels
+    double wsum[9] = {}, lsum = 0.0, bsum = 0.0;
+    for (int tile = blockIdx.x; tile < n; tile += gridDim.x) {
+        {
+            float4 v[4];
+            load_tile(a + (size_t)tile * kC * 256, v);
+            __syncthreads();
+            tile_to_planes(v, planes);
+        }
+        __syncthreads();
+        {
+            float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const float* x = planes + (4 * grp + i) * kPlane + sr * kRow + sc;
+                const float* wr = ws + (4 * grp + i) * 12;
+#pragma unroll
+                for (int ky = 0; ky < 3; ++ky) {
+                    float v[6];
+#pragma unroll
+                    for (int k = 0; k < 3; ++k) {
+                        const float2 z = *reinterpret_cast<const float2*>(x + ky * kRow + 2 * k);
+                        v[2 * k] = z.x;
+                        v[2 * k + 1] = z.y;
+                    }
+#pragma unroll
+                    for (int kx = 0; kx < 3; ++kx)
+#pragma unroll
+                        for (int e = 0; e < 4; ++e)
+                            acc[e] = fmaf(wr[3 * ky + kx], v[e + kx], acc[e]);
+                }
+            }
+            *reinterpret_cast<float4*>(part + grp * 256 + sr * 16 + sc) =
+                make_float4(acc[0], acc[1], acc[2], acc[3]);
+        }
+        __syncthreads();
+        if (t < 256) {
+            float y = bias;
+#pragma unroll
+            for (int k = 0; k < 8; ++k) y += part[k * 256 + t];
+            const float d = y - __ldg(target + (size_t)tile * 256 + t);
+            const float gy = (float)(2.0 * inv * (double)d);
+            lsum += (double)d * d;
+            bsum += (double)gy;
+            gp[((t >> 4) + 1) * kRow + (t & 15) + 1] = gy;
+        }
+        __syncthreads();
+        {  // input gradient: strip of 4 pixels, 4 channels
+            float v[3][6];
+#pragma unroll
+            for (int k = 0; k < 9; ++k) {
+                const float2 z = *reinterpret_cast<const float2*>(gp + (sr + k / 3) * kRow + sc +
+                                                                  2 * (k % 3));
+                v[k / 3][2 * (k % 3)] = z.x;
+                v[k / 3][2 * (k % 3) + 1] = z.y;
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int ci = 4 * grp + i;
+                const float* wr = ws + ci * 12;
+                float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+                for (int k = 0; k < 9; ++k)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e)
+                        acc[e] = fmaf(wr[8 - k], v[k / 3][e + k % 3], acc[e]);
+                const float* x = planes + ci * kPlane + (sr + 1) * kRow + sc + 1;
+                *reinterpret_cast<float4*>(g + (size_t)tile * kC * 256 + ci * 256 + sr * 16 + sc) =
+                    make_float4(x[0] > 0.0f ? acc[0] : 0.0f, x[1] > 0.0f ? acc[1] : 0.0f,
+                                x[2] > 0.0f ? acc[2] : 0.0f, x[3] > 0.0f ? acc[3] : 0.0f);
+            }
+        }
+        {  // weight gradient: lane = input channel, warp = row
+            float gr[16], acc[9];
+#pragma unroll
+            for (int c = 0; c < 16; ++c) gr[c] = gp[(w + 1) * kRow + c + 1];
+#pragma unroll
+            for (int ky = 0; ky < 3; ++ky) {
+                const float* x = planes + lane * kPlane + (w + ky) * kRow;
+                float v[18];
+#pragma unroll
+                for (int q = 0; q < 9; ++q) {
+                    const float2 z = *reinterpret_cast<const float2*>(x + 2 * q);
+                    v[2 * q] = z.x;
+                    v[2 * q + 1] = z.y;
+                }
+#pragma unroll
+                for (int kx = 0; kx < 3; ++kx) {
+                    float s = 0.0f;
+#pragma unroll
+                    for (int c = 0; c < 16; ++c) s = fmaf(gr[c], v[c + kx], s);
+                    acc[3 * ky + kx] = s;
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < 9; ++k) wsum[k] += (double)acc[k];
+        }
+    }
+    // one atomic per value and CTA
+    __syncthreads();
+    double* all = reinterpret_cast<double*>(planes);  // [warp][9][ci]
+#pragma unroll
+    for (int k = 0; k < 9; ++k) all[(w * 9 + k) * kC + lane] = wsum[k];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        lsum += __shfl_xor_sync(0xffffffffu, lsum, o);
+        bsum += __shfl_xor_sync(0xffffffffu, bsum, o);
+    }
+    if (lane == 0) {
+        red[w] = lsum;
+        red[16 + w] = bsum;
+    }
+    __syncthreads();
+    for (int i = t; i < 9 * kC; i += kThreads) {
+        double s = 0.0;
+        for (int k = 0; k < 16; ++k) s += all[k * 9 * kC + i];
+        atomicAdd(dwt + (i % kC) * 9 + i / kC, (float)s);
+    }
+    if (t == 0) {
+        double l = 0.0, s = 0.0;
+        for (int k = 0; k < 8; ++k) {
+            l += red[k];
+            s += red[16 + k];
+        }
+        atomicAdd(loss, (float)(l * inv));
+        atomicAdd(db, (float)s);
     }
 }
 

@@ -214,52 +214,60 @@ class WarmStartNet:
                         "ncsb_net_features")
         return x, sc
 
+    def _param_ptrs(self, vec):
+        """(weights, bias) of each layer in a packed vector, as C pointers."""
+        p = vec.data_ptr()
+        return [(ctypes.c_void_p(p + 4 * wo), ctypes.c_void_p(p + 4 * bo))
+                for wo, _, bo, _ in layer_offsets()]
+
+    def _conv(self, x, layer, sp):
+        """One layer's output on x (in the layer's own buffer)."""
+        cin, cout, relu = LAYERS[layer]
+        n = x.shape[0]
+        y = self._buf("a%d" % layer, (n, cout, 16, 16))
+        w, b = self._param_ptrs(self.params)[layer]
+        self._check(self.lib.ncsb_net_conv_fwd(_ptr(x), w, b, _ptr(y), n, cin, cout, int(relu), sp),
+                    "ncsb_net_conv_fwd")
+        return y
+
+    def _hidden(self, x, sp):
+        """Outputs [a1, a2, a3] of the hidden layers."""
+        acts = []
+        for layer in range(3):
+            acts.append(self._conv(acts[-1] if acts else x, layer, sp))
+        return acts
+
     def forward(self, x):
         """Layer outputs [a1, a2, a3, y] of the network on features x."""
-        n = x.shape[0]
-        acts, cur = [], x
         sp = _stream_ptr(None, self.device)
-        for li, ((w, b), (cin, cout, relu)) in enumerate(zip(self._slices(self.params), LAYERS)):
-            y = self._buf("a%d" % li, (n, cout, 16, 16))
-            self._check(self.lib.ncsb_net_conv_fwd(_ptr(cur), _ptr(w), _ptr(b), _ptr(y), n, cin,
-                                                   cout, int(relu), sp), "ncsb_net_conv_fwd")
-            acts.append(y)
-            cur = y
-        return acts
+        acts = self._hidden(x, sp)
+        return acts + [self._conv(acts[-1], 3, sp)]
 
     def loss_and_grad(self, x, target):
         """MSE loss and its gradient [N_PARAMS] for features x and target y*."""
         n = x.shape[0]
         sp = _stream_ptr(None, self.device)
         with torch.cuda.device(self.device):
-            acts = self.forward(x)
-            grad = self._buf("grad", (N_PARAMS,))
-            grad.zero_()
-            loss = self._buf("loss", (1,))
-            loss.zero_()
-            gy = self._buf("g3", (n, 1, 16, 16))
-            self._check(self.lib.ncsb_net_mse_grad(_ptr(acts[3]), _ptr(target), _ptr(gy),
-                                                   _ptr(loss), n * 256, sp), "ncsb_net_mse_grad")
-            gslices = self._slices(grad)
-            wslices = self._slices(self.params)
-            g = gy
-            for li in range(3, -1, -1):
-                cin, cout, _ = LAYERS[li]
-                inp = acts[li - 1] if li > 0 else x
-                dw, db = gslices[li]
-                self._check(self.lib.ncsb_net_conv_wgrad(_ptr(inp), _ptr(g), _ptr(dw), _ptr(db),
-                                                         n, cin, cout, sp), "ncsb_net_conv_wgrad")
-                if li == 0:
-                    break
-                wf = self._buf("wf%d" % li, (cin * 9 * cout,))
-                self._check(self.lib.ncsb_net_flip(_ptr(wslices[li][0]), _ptr(wf), cin, cout, sp),
-                            "ncsb_net_flip")
-                gx = self._buf("g%d" % (li - 1), (n, cin, 16, 16))
-                self._check(self.lib.ncsb_net_conv_fwd(_ptr(g), _ptr(wf), None, _ptr(gx), n, cout,
-                                                       cin, 0, sp), "ncsb_net_conv_fwd")
-                self._check(self.lib.ncsb_net_relu_bwd(_ptr(gx), _ptr(inp), gx.numel(), sp),
-                            "ncsb_net_relu_bwd")
-                g = gx
+            a1, a2, a3 = self._hidden(x, sp)
+            out = self._buf("loss_grad", (N_PARAMS + 1,))  # the gradient, then the loss
+            out.zero_()
+            grad, loss = out[:N_PARAMS], out[N_PARAMS:]
+            ptr, base = self._param_ptrs(self.params), self._param_ptrs(grad)
+            (_, _), (w2, _), (w3, _), (w4, b4) = ptr
+            (d1, e1), (d2, e2), (d3, e3), (d4, e4) = base
+            lib = self.lib
+            g3 = self._buf("g2", (n, C, 16, 16))
+            self._check(lib.ncsb_net_last_layer(_ptr(a3), w4, b4, _ptr(target), _ptr(g3), d4, e4,
+                                                _ptr(loss), n, sp), "ncsb_net_last_layer")
+            self._check(lib.ncsb_net_conv_wgrad(_ptr(a2), _ptr(g3), d3, e3, n, C, C, sp),
+                        "ncsb_net_conv_wgrad")
+            g2 = self._buf("g1", (n, C, 16, 16))
+            self._check(lib.ncsb_net_conv_xgrad(_ptr(g3), w3, _ptr(a2), _ptr(g2), n, sp),
+                        "ncsb_net_conv_xgrad")
+            self._check(lib.ncsb_net_conv_wgrad(_ptr(a1), _ptr(g2), d2, e2, n, C, C, sp),
+                        "ncsb_net_conv_wgrad")
+            self._check(lib.ncsb_net_first_layers_grad(_ptr(g2), w2, _ptr(a1), _ptr(x), d1, e1, n,
+                                                       sp), "ncsb_net_first_layers_grad")
         return loss, grad
 
     def adam_step(self, grad, lr=1e-3, b1=0.9, b2=0.999, eps=1e-8):
