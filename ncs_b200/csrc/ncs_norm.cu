@@ -9,9 +9,9 @@
 //
 // One thread per pixel: 9 unknowns, FP64 iterate, gradient and costs (the
 // cost is a sum of terms of order 100 whose differences near convergence are
-// of order 1e-5), BFGS with a dense 9 x 9 inverse-Hessian approximation kept
-// in shared memory (45 packed FP32 entries per thread; the direction and the
-// update in FP32 as the main solver's L-BFGS, the update's scalars in FP64),
+// of order 1e-5), BFGS with a dense 9 x 9 inverse-Hessian approximation (45
+// packed FP32 entries per thread; the direction and the update in FP32 as the
+// main solver's L-BFGS, the update's scalars in FP64),
 // backtracking Armijo line search on the FP64 cost change (in difference
 // form, see the trial loop) with the fraction-to-barrier rule of the main
 // solver.  The
@@ -21,6 +21,16 @@
 // 3 x 3 circular convolution with the kernel qk = ifft2(M^2) / 9 (block
 // circulant with circulant blocks): Q[p][q] = qk[(p1 - q1) mod 3][(p2 - q2)
 // mod 3], so the kernel takes 9 values from the host instead of 45.
+//
+// What bounds it: instruction issue and FP64 latency at 8 warps per SM, and
+// divergence -- a warp runs until its slowest pixel, 1.4 times the mean count.
+// 20 frames of 512^2 take 3.38 ms: 3.74 with separate FP64 comparisons for the
+// step's range, the barrier and the stopping test instead of integer maxima of
+// upper words, and s = un - u instead of the FP32 step itself; 4.13 with two
+// quadratic instead of one cubic refinement of each reciprocal; 4.82 also with
+// Q u as 81 products and two reciprocals per pixel and trial.  Refilling a
+// warp's finished lanes with new pixels ran 4.2 ms: first iterations, which
+// backtrack, then hold up a warp all the time instead of once.
 #include <cuda_runtime.h>
 #include <math_constants.h>
 #include <stdint.h>
@@ -30,9 +40,13 @@
 namespace ncsb {
 namespace norm {
 
-// 64 threads a block: the inverse Hessians (45 x 4 B a thread) and segment
-// constants take 20 KB of static shared memory
+// 64 threads a block: three FP64 vectors (216 B a thread) take 14 KB of static
+// shared memory
 constexpr int kThreads = 64;
+// blocks per SM: 4 (8 warps) with the inverse Hessian and the iterate's vectors
+// in registers.  6 blocks (168 registers) with them re-read from shared memory
+// ran 4 % slower, and spilled them 30 %.
+constexpr int kBlocks = 4;
 constexpr int kPacked = 45;  // upper triangle of a symmetric 9 x 9
 
 struct Args {
@@ -54,169 +68,178 @@ __host__ __device__ constexpr int pk(int i, int j) {  // packed index, i <= j
 }
 
 
-// Per-thread constants of the segment in shared memory (c = d + gamma, gamma),
-// column t of each [9][kThreads] array.
-struct Seg {
-    const double (*c)[kThreads];
-    const double (*gm)[kThreads];
-    int t;
-    __device__ double C(int i) const { return c[i][t]; }
-    __device__ double G(int i) const { return gm[i][t]; }
-};
-
 // Q u, S = sum u and P = u'Q u at a point (the noise term is alpha P / S).
-__device__ void noise_parts(const Args& a, const double (&u)[9], double (&Qu)[9], double& S,
-                            double& P) {
-    S = 0.0;
-    P = 0.0;
+// Quad: the mask has M(k1, k2) = M(k1, -k2), so qk has four distinct values and
+// Q u comes from the segment's row, column and total sums (29 additions and
+// multiply-adds instead of 81).
+template <bool Quad>
+__device__ __forceinline__ void noise_parts(const Args& a, const double (&u)[9], double (&Qu)[9],
+                                            double& S, double& P) {
+    if constexpr (Quad) {
+        const double q0 = a.qk[0], qr = a.qk[1], qc = a.qk[3], qd = a.qk[4];
+        double R[3], C[3];
 #pragma unroll
-    for (int i = 0; i < 9; ++i) {
-        S += u[i];
-        double acc = 0.0;
+        for (int k = 0; k < 3; ++k) {
+            R[k] = (u[3 * k] + u[3 * k + 1]) + u[3 * k + 2];
+            C[k] = (u[k] + u[k + 3]) + u[k + 6];
+        }
+        S = (R[0] + R[1]) + R[2];
+        const double dS = qd * S, kr = qr - qd, kc = qc - qd, ku = (q0 - qr) - kc;
 #pragma unroll
-        for (int j = 0; j < 9; ++j)
-            acc = fma(a.qk[((i / 3 - j / 3 + 3) % 3) * 3 + (i % 3 - j % 3 + 3) % 3], u[j], acc);
-        Qu[i] = acc;
+        for (int k = 0; k < 3; ++k) {
+            R[k] = fma(kr, R[k], dS);
+            C[k] = kc * C[k];
+        }
+#pragma unroll
+        for (int i = 0; i < 9; ++i) Qu[i] = fma(ku, u[i], R[i / 3] + C[i % 3]);
+    } else {
+        S = 0.0;
+#pragma unroll
+        for (int i = 0; i < 9; ++i) {
+            S += u[i];
+            double acc = 0.0;
+#pragma unroll
+            for (int j = 0; j < 9; ++j)
+                acc = fma(a.qk[((i / 3 - j / 3 + 3) % 3) * 3 + (i % 3 - j % 3 + 3) % 3], u[j], acc);
+            Qu[i] = acc;
+        }
     }
+    P = 0.0;
 #pragma unroll
     for (int i = 0; i < 9; ++i) P = fma(u[i], Qu[i], P);
 }
 
 // 1/x for x > 0: the hardware's gross FP64 reciprocal (PTX rcp.approx.ftz.f64,
-// from the operand's upper 32 bits) refined by two Newton steps r (2 - x r),
-// each of which squares the relative error, to FP64 rounding.  No FP32
+// from the operand's upper 32 bits, about 20 bits) refined by one third-order
+// step r (1 + e + e^2), e = 1 - x r, which cubes the relative error.  No FP32
 // round trip: conversions share the pipe with the reciprocal itself.
 __device__ __forceinline__ double recip(double x) {
     double r;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
-    r = r * fma(-x, r, 2.0);
-    return r * fma(-x, r, 2.0);
+    const double e = fma(-x, r, 1.0);
+    return fma(r, fma(e, e, e), r);
 }
 
-// log1p(x) for |x| <= kSeriesMax: 2 atanh(y), y = x / (2 + x), |y| < 0.18, by
-// the odd series 2y (1 + y^2/3 + ... + y^14/15); the first omitted term,
-// y^16/17, is below 6e-14 relative, and y carries the reciprocal's 2^-46.
-constexpr double kSeriesMax = 0.3;
-__device__ __forceinline__ double log1p_series(double x) {
-    const double y = x * recip(2.0 + x), y2 = y * y;
-    double s = fma(y2, 1.0 / 15.0, 1.0 / 13.0);
-    s = fma(y2, s, 1.0 / 11.0);
-    s = fma(y2, s, 1.0 / 9.0);
-    s = fma(y2, s, 1.0 / 7.0);
-    s = fma(y2, s, 1.0 / 5.0);
-    s = fma(y2, s, 1.0 / 3.0);
-    s = fma(y2, s, 1.0);
-    return 2.0 * y * s;
+// log1p(x) for |x| <= 0.3 is 2 atanh(y), y = x / (2 + x), |y| < 0.18;
+// 2 atanh(y) / y as a polynomial in y^2, minimax in relative error (4e-14).
+constexpr int kSeriesHi = 0x3fd33333;  // upper word of 0.3
+__device__ __forceinline__ double atanh2_poly(double y2) {
+    double s = fma(y2, 0.19696279890493262, 0.2216823319916572);
+    s = fma(y2, s, 0.2857230812738637);
+    s = fma(y2, s, 0.3999999354479562);
+    s = fma(y2, s, 0.6666666668396458);
+    return fma(y2, s, 1.999999999999925);
 }
 
-// the cost at u (FP64 logs; once per pixel, for the reported cost)
-__device__ double full_cost(const Args& a, const double (&u)[9], const Seg& sg) {
-    double Qu[9], S, P, ll = 0.0;
-    noise_parts(a, u, Qu, S, P);
+// |x| as its upper 32 bits: ordered as |x| up to 2^-20 relative (NaN above all)
+__device__ __forceinline__ int abs_hi(double x) { return __double2hiint(x) & 0x7fffffff; }
+
+// x[i] of a register array at a runtime index
+template <typename T>
+__device__ __forceinline__ T pick(const T (&x)[9], int i) {
+    T v = x[0];
 #pragma unroll
-    for (int i = 0; i < 9; ++i) ll += u[i] - sg.C(i) * log(u[i] + sg.G(i));
-    return (2.0 / 9.0) * ll + a.alpha * P / S;
+    for (int k = 1; k < 9; ++k) v = i == k ? x[k] : v;
+    return v;
 }
 
-// gradient at u from its noise parts and r_i = 1 / (u_i + gamma_i)
-__device__ void gradient(const Args& a, const double (&Qu)[9], double S, double P,
-                         const double (&r)[9], const Seg& sg, double (&g)[9]) {
-    const double is = recip(S), is2 = is * is;
-#pragma unroll
-    for (int i = 0; i < 9; ++i)
-        g[i] = (2.0 / 9.0) * (1.0 - sg.C(i) * r[i]) + a.alpha * (2.0 * Qu[i] * S - P) * is2;
-}
-
-__global__ void __launch_bounds__(kThreads) normalized_kernel(const Args a) {
-    __shared__ float Hm[kPacked][kThreads];  // inverse-Hessian approximation, per thread
-    __shared__ double Cs[9][kThreads], Gs[9][kThreads];
+template <bool Quad>
+__global__ void __launch_bounds__(kThreads, kBlocks) normalized_kernel(const Args a) {
+    __shared__ double Cs[9][kThreads];  // (2/9) (d + gamma)
     __shared__ double Rs[9][kThreads];  // 1 / (u + gamma) at the current iterate
+    __shared__ double Gs[9][kThreads];  // the gradient there
     const long long HW = (long long)a.H * a.W;
     const long long idx = (long long)blockIdx.x * kThreads + threadIdx.x;
     if (idx >= (long long)a.T * HW) return;
-    const int f = (int)(idx / HW);
-    const long long p = idx - (long long)f * HW;
-    const int y = (int)(p / a.W), x = (int)(p - (long long)y * a.W);
-    const float* img = a.data + (long long)f * HW;
-    const float* gmap = a.gamma + (long long)f * a.gstride;
     const int t = threadIdx.x;
-    double u[9], g[9];
+    // the segment's data and gamma (replicate-padded)
+    auto segment = [&](double (&d)[9], double (&gm)[9]) {
+        const int f = (int)(idx / HW);
+        const long long p = idx - (long long)f * HW;
+        const int y = (int)(p / a.W), x = (int)(p - (long long)y * a.W);
+        const float* img = a.data + (long long)f * HW;
+        const float* gmap = a.gamma + (long long)f * a.gstride;
 #pragma unroll
-    for (int r = 0; r < 3; ++r) {
-        const int yy = min(max(y + r - 1, 0), a.H - 1);
+        for (int r = 0; r < 3; ++r) {
+            const int yy = min(max(y + r - 1, 0), a.H - 1);
 #pragma unroll
-        for (int s = 0; s < 3; ++s) {
-            const int xx = min(max(x + s - 1, 0), a.W - 1);
-            const double dv = img[(long long)yy * a.W + xx];
-            const double gv = gmap[(long long)yy * a.W + xx];
-            u[3 * r + s] = dv;
-            Gs[3 * r + s][t] = gv;
-            Cs[3 * r + s][t] = dv + gv;
+            for (int s = 0; s < 3; ++s) {
+                const int xx = min(max(x + s - 1, 0), a.W - 1);
+                d[3 * r + s] = img[(long long)yy * a.W + xx];
+                gm[3 * r + s] = gmap[(long long)yy * a.W + xx];
+            }
         }
-    }
-    const Seg sg{Cs, Gs, t};
-#pragma unroll
-    for (int i = 0; i < 9; ++i)
-#pragma unroll
-        for (int j = i; j < 9; ++j) Hm[pk(i, j)][t] = i == j ? 1.0f : 0.0f;
-
-    double Qu[9], S, P;
-    noise_parts(a, u, Qu, S, P);
-    bool feasible = S > 0.0;
+    };
+    double u[9], g_stop = 0.0, fq = 0.0, res_f = 0.0;
+    float gf[9], H[kPacked];  // gradient, inverse-Hessian approximation
+    int status = 0, it = 0, g_hi = 0, stop_hi = 0;
+    bool feasible;
     {
-        double r[9];
+        double gm[9], Qu[9], S, P, g0 = 0.0;
+        segment(u, gm);
+        noise_parts<Quad>(a, u, Qu, S, P);
+        feasible = S > 0.0;
 #pragma unroll
-        for (int i = 0; i < 9; ++i) {
-            const double A = u[i] + sg.G(i);
-            feasible = feasible && A > 0.0;
-            r[i] = recip(A > 0.0 ? A : 1.0);
-            Rs[i][t] = r[i];
-        }
-        gradient(a, Qu, S, P, r, sg, g);
-    }
-    double fq = feasible ? P * recip(S) : 0.0;  // P / S at the current iterate
-    // A trial whose cost change is below the cost's FP64 resolution is accepted,
-    // as when two full costs compare equal: near the optimum the gradient still
-    // steers the steps (its test can need changes far below that resolution),
-    // and a step that moves no pixel ends the solve.  The resolution is taken
-    // as 2^-52 of a bound on |f|, (2/9) sum (|u| + c |log(u + gamma)|) +
-    // alpha |P / S|, from the start (FP32 hardware log2: only its scale matters)
-    double res_f = 0.0;
-    if (feasible) {
+        for (int i = 0; i < 9; ++i) feasible = feasible && u[i] + gm[i] > 0.0;
+        const double is = recip(S);
+        fq = feasible ? P * is : 0.0;  // P / S at the current iterate
+        // A trial whose cost change is below the cost's FP64 resolution is
+        // accepted, as when two full costs compare equal: near the optimum the
+        // gradient still steers the steps (its test can need changes far below
+        // that resolution), and a step that moves no pixel ends the solve.  The
+        // resolution is taken as 2^-52 of a bound on |f|, (2/9) sum (|u| +
+        // c |log(u + gamma)|) + alpha |P / S|, from the start (FP32 hardware
+        // log2: only its scale matters)
         float bound = 0.0f;
+        const double k1 = 2.0 * a.alpha * is, k0 = fma(-a.alpha * P * is, is, 2.0 / 9.0);
 #pragma unroll
         for (int i = 0; i < 9; ++i) {
+            const double A = u[i] + gm[i], c = A;  // u = d: c = d + gamma
+            const double r = recip(A > 0.0 ? A : 1.0);
+            Cs[i][t] = (2.0 / 9.0) * c;
+            Rs[i][t] = r;
+            const double g = fma(k1, Qu[i], fma(-(2.0 / 9.0) * c, r, k0));
+            Gs[i][t] = g;
+            gf[i] = (float)g;
+            g0 = fmax(g0, fabs(g));
+            g_hi = max(g_hi, abs_hi(g));
             float l2;
-            asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(l2) : "f"((float)(u[i] + sg.G(i))));
-            bound += fabsf((float)u[i]) + (float)sg.C(i) * fabsf(l2 * 0.69314718f);
+            asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(l2) : "f"((float)A));
+            bound += fabsf((float)u[i]) + (float)c * fabsf(l2 * 0.69314718f);
         }
         res_f = 0x1p-52 * ((2.0 / 9.0) * (double)bound + a.alpha * fabs(fq));
+#pragma unroll
+        for (int i = 0; i < 9; ++i)
+#pragma unroll
+            for (int j = i; j < 9; ++j) H[pk(i, j)] = i == j ? 1.0f : 0.0f;
+        g_stop = a.tol * fmax(1.0, g0);
+        stop_hi = abs_hi(g_stop);
     }
-    double g0 = 0.0;
+    status = feasible ? NCSB_REACHED_MAXITERS : NCSB_INCREASING_GRADIENT;
+    while (feasible && it < a.max_iters) {
+        // some |g_i| above the stopping threshold, by the upper words unless these
+        // leave it open
+        bool steep = g_hi > stop_hi && g_hi < 0x7ff00000;
+        if (!steep && g_hi >= stop_hi) {
 #pragma unroll
-    for (int i = 0; i < 9; ++i) g0 = fmax(g0, fabs(g[i]));
-    int status = NCSB_REACHED_MAXITERS, it = 0;
-    if (!feasible) status = NCSB_INCREASING_GRADIENT;  // infeasible start
-    for (; it < a.max_iters && status == NCSB_REACHED_MAXITERS; ++it) {
-        double gmax = 0.0;
-#pragma unroll
-        for (int i = 0; i < 9; ++i) gmax = fmax(gmax, fabs(g[i]));
-        if (gmax <= a.tol * fmax(1.0, g0)) { status = NCSB_SUCCESS; break; }
+            for (int i = 0; i < 9; ++i) steep = steep || fabs(Gs[i][t]) > g_stop;
+        }
+        if (!steep) {
+            status = NCSB_SUCCESS;
+            break;
+        }
         // direction p = -H g and its slope g'p = -g'H g, both FP32 (a quadratic
         // form: no cancellation; the Armijo threshold needs it to 1e-4 at most)
         float d[9];
         double gd;
-        float gf[9];
         {
             float gdf = 0.0f;
-#pragma unroll
-            for (int j = 0; j < 9; ++j) gf[j] = (float)g[j];
 #pragma unroll
             for (int i = 0; i < 9; ++i) {
                 float acc = 0.0f;
 #pragma unroll
                 for (int j = 0; j < 9; ++j)
-                    acc = fmaf(Hm[i <= j ? pk(i, j) : pk(j, i)][t], gf[j], acc);
+                    acc = fmaf(H[i <= j ? pk(i, j) : pk(j, i)], gf[j], acc);
                 d[i] = -acc;
                 gdf = fmaf(gf[i], d[i], gdf);
             }
@@ -226,7 +249,7 @@ __global__ void __launch_bounds__(kThreads) normalized_kernel(const Args a) {
 #pragma unroll
             for (int i = 0; i < 9; ++i)
 #pragma unroll
-                for (int j = i; j < 9; ++j) Hm[pk(i, j)][t] = i == j ? 1.0f : 0.0f;
+                for (int j = i; j < 9; ++j) H[pk(i, j)] = i == j ? 1.0f : 0.0f;
             float gdf = 0.0f;
 #pragma unroll
             for (int i = 0; i < 9; ++i) {
@@ -236,74 +259,100 @@ __global__ void __launch_bounds__(kThreads) normalized_kernel(const Args a) {
             gd = (double)gdf;
         }
         // backtracking Armijo on the cost change in difference form:
-        //   f(un) - f(u) = (2/9) sum_i [s_i - c_i log1p(s_i / (u_i + gamma_i))]
-        //                  + alpha (P(un) / S(un) - P(u) / S(u)),  s = un - u,
-        // whose log terms are of the order of the step rather than of the costs
-        // (about 100), so a series log1p at 1e-13 replaces the FP64 logs of two
-        // full costs; trials keep u + gamma >= 1% of its value
-        double step = 1.0, un[9], gn[9], Qn[9], Sn = 0.0, Pn = 0.0, fqn = 0.0, df = 0.0;
+        //   f(un) - f(u) = (2/9) sum_i [s_i - c_i log1p(x_i)]
+        //                  + alpha (P(un) / S(un) - P(u) / S(u)),
+        // s the step d (FP32 values), x_i = s_i / (u_i + gamma_i), whose log terms
+        // are of the order of the step rather than of the costs (about 100), so a
+        // polynomial log1p at 4e-14 replaces the FP64 logs of two full costs.  Trials
+        // keep u + gamma >= 1% of its value: x >= -0.99.  One reciprocal, of
+        // (1 + x)(2 + x), gives y = x / (2 + x) of the log1p and 1 / (un + gamma) =
+        // (1 / (u + gamma)) / (1 + x) of the next gradient.
+        double step = 1.0, un[9], Qn[9], rn[9], Sn = 0.0, Pn = 0.0, isn = 0.0, fqn = 0.0;
         bool ok = false;
+        int x_hi = 0;  // max |x|
         for (int trial = 0; trial < 64; ++trial) {
-            bool feas = true;
+#pragma unroll
+            for (int i = 0; i < 9; ++i) un[i] = u[i] + (double)d[i];
+            x_hi = 0;
+            double ssum = 0.0, lsum = 0.0;
 #pragma unroll
             for (int i = 0; i < 9; ++i) {
-                un[i] = fma(step, (double)d[i], u[i]);
-                feas = feas && (un[i] + sg.G(i) >= 0.01 * (u[i] + sg.G(i)));
+                const double s = d[i], r = Rs[i][t], x = s * r;
+                x_hi = max(x_hi, abs_hi(x));
+                const double x1 = 1.0 + x, x2 = 2.0 + x, q = recip(x1 * x2);
+                const double y = x * (q * x1);
+                rn[i] = r * (q * x2);
+                ssum += s;
+                lsum = fma(Cs[i][t], y * atanh2_poly(y * y), lsum);
+            }
+            noise_parts<Quad>(a, un, Qn, Sn, Pn);
+            bool feas = Sn > 0.0;
+            if (x_hi >= kSeriesHi) {  // a relative step beyond the series' range
+                lsum = 0.0;
+#pragma unroll 1
+                for (int i = 0; i < 9; ++i) {
+                    const double x = (double)pick(d, i) * Rs[i][t];
+                    feas = feas && x >= -0.99;
+                    lsum = fma(Cs[i][t], log1p(x), lsum);
+                }
             }
             if (feas) {
-                noise_parts(a, un, Qn, Sn, Pn);
-                if (Sn > 0.0) {
-                    double dll = 0.0;
-                    bool big = false;
-#pragma unroll
-                    for (int i = 0; i < 9; ++i) {
-                        const double si = un[i] - u[i], x = si * Rs[i][t];
-                        big = big || !(fabs(x) <= kSeriesMax);
-                        dll += fma(-sg.C(i), log1p_series(x), si);
-                    }
-                    if (big) {  // a relative step beyond the series' range
-                        dll = 0.0;
-#pragma unroll
-                        for (int i = 0; i < 9; ++i) {
-                            const double si = un[i] - u[i];
-                            dll += fma(-sg.C(i), log1p(si * Rs[i][t]), si);
-                        }
-                    }
-                    fqn = Pn * recip(Sn);  // the same rounding as fq's
-                    df = (2.0 / 9.0) * dll + a.alpha * (fqn - fq);
-                    if (df <= a.c1 * step * gd || fabs(df) <= res_f) {
-                        ok = true;
-                        break;
-                    }
+                isn = recip(Sn);
+                fqn = Pn * isn;  // the same rounding as fq's
+                const double df = fma(2.0 / 9.0, ssum, -lsum) + a.alpha * (fqn - fq);
+                if (df <= a.c1 * step * gd || fabs(df) <= res_f) {
+                    ok = true;
+                    break;
                 }
             }
             step *= 0.5;
             if (!(step >= a.min_step)) break;
-        }
-        if (!ok) { status = NCSB_MINIMUM_STEP; break; }
-        double rn[9];  // un + gamma >= 1% of u + gamma > 0
 #pragma unroll
-        for (int i = 0; i < 9; ++i) rn[i] = recip(un[i] + sg.G(i));
-        gradient(a, Qn, Sn, Pn, rn, sg, gn);
-        // BFGS update of the inverse Hessian with s = un - u, y = gn - g:
+            for (int i = 0; i < 9; ++i) d[i] *= 0.5f;
+        }
+        if (!ok) {
+            status = NCSB_MINIMUM_STEP;
+            break;
+        }
+        // BFGS update of the inverse Hessian with s = d, y = gn - g:
         // H <- H - rho (v s' + s v') + (rho^2 y'Hy + rho) s s', v = H y.  The
         // differences and the scalars in FP64, the 45 entries in FP32 from
         // pre-scaled vectors (no FP32 product of rho or rho^2 alone).
-        float s[9], yv[9];
+        float yv[9];
         double sy = 0.0, yy = 0.0;
+        g_hi = 0;
+        if ((it & 15) == 15) {  // against the drift of the products above
+            double dat[9], gm[9];
+            segment(dat, gm);
+#pragma unroll
+            for (int i = 0; i < 9; ++i) rn[i] = recip(un[i] + gm[i]);
+        }
+        // a step above 2^-50 of u + gamma moves u
+        bool moved = x_hi >= 0x3cd00000;
+        if (!moved) {
+#pragma unroll
+            for (int i = 0; i < 9; ++i) moved = moved || un[i] != u[i];
+        }
+        const double k1 = 2.0 * a.alpha * isn, k0 = fma(-a.alpha * fqn, isn, 2.0 / 9.0);
 #pragma unroll
         for (int i = 0; i < 9; ++i) {
-            const double sd = un[i] - u[i], yd = gn[i] - g[i];
-            s[i] = (float)sd;
+            const double sd = d[i];
+            const double gn = fma(k1, Qn[i], fma(-Cs[i][t], rn[i], k0));
+            const double yd = gn - Gs[i][t];
+            Gs[i][t] = gn;
+            Rs[i][t] = rn[i];
+            u[i] = un[i];
+            gf[i] = (float)gn;
+            g_hi = max(g_hi, abs_hi(gn));
             yv[i] = (float)yd;
             sy = fma(sd, yd, sy);
-            yy = fma(yd, yd, yy);
+            if (it == 0) yy = fma(yd, yd, yy);
         }
         if (sy > 1e-30) {  // rho = 1 / sy within FP32 range
             if (it == 0) {  // scale the identity before the first update
                 const float sc = (float)(sy / yy);
 #pragma unroll
-                for (int i = 0; i < 9; ++i) Hm[pk(i, i)][t] = sc;
+                for (int i = 0; i < 9; ++i) H[pk(i, i)] = sc;
             }
             float v[9], yHyf = 0.0f;
 #pragma unroll
@@ -311,7 +360,7 @@ __global__ void __launch_bounds__(kThreads) normalized_kernel(const Args a) {
                 float acc = 0.0f;
 #pragma unroll
                 for (int j = 0; j < 9; ++j)
-                    acc = fmaf(Hm[i <= j ? pk(i, j) : pk(j, i)][t], yv[j], acc);
+                    acc = fmaf(H[i <= j ? pk(i, j) : pk(j, i)], yv[j], acc);
                 v[i] = acc;
                 yHyf = fmaf(yv[i], acc, yHyf);
             }
@@ -321,33 +370,40 @@ __global__ void __launch_bounds__(kThreads) normalized_kernel(const Args a) {
 #pragma unroll
             for (int i = 0; i < 9; ++i) {
                 rv[i] = rhof * v[i];
-                ks[i] = (float)(k2 * (double)s[i]);
+                ks[i] = (float)(k2 * (double)d[i]);
             }
 #pragma unroll
             for (int i = 0; i < 9; ++i)
 #pragma unroll
                 for (int j = i; j < 9; ++j) {
-                    const float h = Hm[pk(i, j)][t];
-                    Hm[pk(i, j)][t] =
-                        fmaf(ks[i], s[j], fmaf(-rv[i], s[j], fmaf(-s[i], rv[j], h)));
+                    const float h = H[pk(i, j)];
+                    H[pk(i, j)] =
+                        fmaf(ks[i], d[j], fmaf(-rv[i], d[j], fmaf(-d[i], rv[j], h)));
                 }
         }
-        bool moved = false;
-#pragma unroll
-        for (int i = 0; i < 9; ++i) {
-            moved = moved || (un[i] != u[i]);
-            u[i] = un[i];
-            g[i] = gn[i];
-            Rs[i][t] = rn[i];
-        }
         fq = fqn;
-        if (!moved) { status = NCSB_REACHED_MAXPRECISION; ++it; break; }
+        ++it;
+        if (!moved) {
+            status = NCSB_REACHED_MAXPRECISION;
+            break;
+        }
     }
     const float centre = (float)u[4];
     a.out[idx] = centre < 0.0f ? 1.0e-6f : centre;
     if (a.iters) a.iters[idx] = it;
     if (a.status) a.status[idx] = status;
-    if (a.cost) a.cost[idx] = feasible ? full_cost(a, u, sg) : CUDART_INF;
+    if (a.cost) {  // with FP64 logs, once
+        double cost = CUDART_INF;
+        if (feasible) {
+            double d[9], gm[9], Qu[9], S, P, ll = 0.0;
+            segment(d, gm);
+            noise_parts<Quad>(a, u, Qu, S, P);
+#pragma unroll
+            for (int i = 0; i < 9; ++i) ll += u[i] - (d[i] + gm[i]) * log(u[i] + gm[i]);
+            cost = (2.0 / 9.0) * ll + a.alpha * P / S;
+        }
+        a.cost[idx] = cost;
+    }
 }
 
 }  // namespace norm
@@ -379,6 +435,8 @@ int ncsb_reduce_noise_normalized(const float* images, int n_frames, int height, 
     double sym[3][3];
     for (int i = 0; i < 3; ++i)
         for (int j = 0; j < 3; ++j) sym[i][j] = 0.5 * (mu[i][j] + mu[(3 - i) % 3][(3 - j) % 3]);
+    bool quad = true;  // M(k1, k2) = M(k1, -k2)
+    for (int i = 0; i < 3; ++i) quad = quad && sym[i][1] == sym[i][2];
     Args a{};
     const double tw = 2.0 * 3.14159265358979323846 / 3.0;
     // qk[d1][d2] = Q[(d1, d2)][(0, 0)]; Re(e^{+i th_p} e^{-i th_q}) = cos(th_p - th_q)
@@ -405,8 +463,9 @@ int ncsb_reduce_noise_normalized(const float* images, int n_frames, int height, 
     a.status = px_status;
     a.cost = px_cost;
     const long long n = (long long)n_frames * height * width;
-    normalized_kernel<<<(unsigned)((n + kThreads - 1) / kThreads), kThreads, 0,
-                        (cudaStream_t)stream>>>(a);
+    const unsigned grid = (unsigned)((n + kThreads - 1) / kThreads);
+    if (quad) normalized_kernel<true><<<grid, kThreads, 0, (cudaStream_t)stream>>>(a);
+    else normalized_kernel<false><<<grid, kThreads, 0, (cudaStream_t)stream>>>(a);
     return cudaGetLastError() == cudaSuccess ? NCSB_OK : NCSB_ECUDA;
 }
 
