@@ -32,6 +32,7 @@
 #ifndef NCS_B200_H
 #define NCS_B200_H
 
+#include <stddef.h>
 #include <stdint.h>
 
 #ifdef __cplusplus
@@ -100,6 +101,12 @@ void ncsb_default_params(ncsb_params *p);
 /* Create a handle on the current CUDA device; allocates its small device
  * workspace (queue counter, mask tables). */
 int ncsb_create(ncsb_handle **out, const ncsb_params *p);
+/* The same with the handle's device scratch (mask table, work counter) given by
+ * the caller, e.g. from its own caching allocator: at least
+ * NCSB_HANDLE_SCRATCH_BYTES, 16-byte aligned, idle when this is called, and
+ * left alone while the handle exists and its launches run. */
+#define NCSB_HANDLE_SCRATCH_BYTES 2048
+int ncsb_create_with_scratch(ncsb_handle **out, const ncsb_params *p, void *scratch, size_t bytes);
 int ncsb_set_params(ncsb_handle *h, const ncsb_params *p);
 int ncsb_destroy(ncsb_handle *h);
 const char *ncsb_last_error(const ncsb_handle *h);

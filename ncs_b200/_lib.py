@@ -110,10 +110,11 @@ class NcsbCalibration(ctypes.Structure):
 
 
 MAX_STACKS = 65536
+HANDLE_SCRATCH_BYTES = 2048
 
 # Every symbol include/ncs_b200.h declares (checked by the tests).
 EXPORTS = [
-    "ncsb_default_params", "ncsb_create", "ncsb_set_params", "ncsb_destroy", "ncsb_last_error",
+    "ncsb_default_params", "ncsb_create", "ncsb_create_with_scratch", "ncsb_set_params", "ncsb_destroy", "ncsb_last_error",
     "ncsb_set_otf_mask", "ncsb_num_tiles", "ncsb_reduce_noise", "ncsb_solve_tiles",
     "ncsb_reduce_noise_noalloc", "ncsb_reduce_noise_start",
     "ncsb_net_param_count", "ncsb_net_conv_fwd", "ncsb_net_conv_wgrad", "ncsb_net_flip",
@@ -152,6 +153,8 @@ def load():
     lib.ncsb_default_params.restype = None
     lib.ncsb_create.argtypes = [P(vp), P(NcsbParams)]
     lib.ncsb_create.restype = ctypes.c_int
+    lib.ncsb_create_with_scratch.argtypes = [P(vp), P(NcsbParams), vp, ctypes.c_size_t]
+    lib.ncsb_create_with_scratch.restype = ctypes.c_int
     lib.ncsb_set_params.argtypes = [vp, P(NcsbParams)]
     lib.ncsb_set_params.restype = ctypes.c_int
     lib.ncsb_destroy.argtypes = [vp]

@@ -112,6 +112,8 @@ struct ncsb_handle {
     int device = 0;
     int num_sms = 1;
     bool has_mask = false;
+    // Device scratch (NCSB_HANDLE_SCRATCH_BYTES), allocated here or the caller's:
+    bool own_scratch = false;
     float* d_msq = nullptr;                 // [256] M^2/256, natural [kr][kc] order
     unsigned long long* d_queue = nullptr;  // work counter
     int32_t* d_flag = nullptr;              // tensor-core forms: 1 after a wait ran out
@@ -275,31 +277,39 @@ void ncsb_default_params(ncsb_params* p) {
     p->ctas_per_sm = 0;
 }
 
-int ncsb_create(ncsb_handle** out, const ncsb_params* p) {
+int ncsb_create_with_scratch(ncsb_handle** out, const ncsb_params* p, void* scratch,
+                             size_t bytes) {
     if (!out) return NCSB_EINVAL;
     *out = nullptr;
     std::string why;
     int rc = check_params(p, &why);
     if (rc != NCSB_OK) return rc;
+    if (scratch && (bytes < NCSB_HANDLE_SCRATCH_BYTES || (uintptr_t)scratch % 16 != 0))
+        return NCSB_ESCRATCH;
     ncsb_handle* h = new (std::nothrow) ncsb_handle();
     if (!h) return NCSB_EINVAL;
     h->p = *p;
     cudaError_t e = cudaGetDevice(&h->device);
     if (e == cudaSuccess)
         e = cudaDeviceGetAttribute(&h->num_sms, cudaDevAttrMultiProcessorCount, h->device);
-    if (e == cudaSuccess) e = cudaMalloc(&h->d_msq, ncsb::kPix * sizeof(float));
-    if (e == cudaSuccess) e = cudaMalloc(&h->d_queue, sizeof(unsigned long long));
-    if (e == cudaSuccess) e = cudaMalloc(&h->d_flag, sizeof(int32_t));
-    if (e == cudaSuccess) e = cudaMemset(h->d_flag, 0, sizeof(int32_t));
+    if (e == cudaSuccess && !scratch) {
+        e = cudaMalloc(&scratch, NCSB_HANDLE_SCRATCH_BYTES);
+        h->own_scratch = e == cudaSuccess;
+    }
     if (e != cudaSuccess) {
-        cudaFree(h->d_msq);
-        cudaFree(h->d_queue);
-        cudaFree(h->d_flag);
         delete h;
         return NCSB_ECUDA;
     }
+    unsigned char* base = static_cast<unsigned char*>(scratch);
+    h->d_msq = reinterpret_cast<float*>(base);
+    h->d_queue = reinterpret_cast<unsigned long long*>(base + ncsb::kPix * sizeof(float));
+    h->d_flag = reinterpret_cast<int32_t*>(base + ncsb::kPix * sizeof(float) + 16);
     *out = h;
     return NCSB_OK;
+}
+
+int ncsb_create(ncsb_handle** out, const ncsb_params* p) {
+    return ncsb_create_with_scratch(out, p, nullptr, 0);
 }
 
 int ncsb_set_params(ncsb_handle* h, const ncsb_params* p) {
@@ -315,9 +325,7 @@ int ncsb_destroy(ncsb_handle* h) {
     if (!h) return NCSB_EINVAL;
     destroy_pipe(h->pipe);
     cudaFree(h->d_adu);
-    cudaFree(h->d_msq);
-    cudaFree(h->d_queue);
-    cudaFree(h->d_flag);
+    if (h->own_scratch) cudaFree(h->d_msq);
     cudaFree(h->d_stacks);
     cudaFree(h->d_mk_lane);
     delete h;

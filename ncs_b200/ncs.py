@@ -37,7 +37,24 @@ def checkOTFMask(otf_mask):
 
 
 def _ptr(t):
-    return ctypes.c_void_p(t.data_ptr()) if t is not None else ctypes.c_void_p(0)
+    return t.data_ptr() if t is not None else None
+
+
+class _on_device:
+    """torch.cuda.device, entered only where the device is not current."""
+
+    __slots__ = ("ctx",)
+
+    def __init__(self, device):
+        self.ctx = None if torch.cuda.current_device() == device.index else torch.cuda.device(device)
+
+    def __enter__(self):
+        if self.ctx is not None:
+            self.ctx.__enter__()
+
+    def __exit__(self, *exc):
+        if self.ctx is not None:
+            self.ctx.__exit__(*exc)
 
 
 def launch_stream(stream, device, *tensors):
@@ -88,8 +105,16 @@ class Solver:
         self._handle = ctypes.c_void_p()
         self._set(alpha=alpha, max_iters=max_iters, m=m, epsilon=epsilon, c1=c1,
                   min_step=min_step, mode=mode, ctas_per_sm=ctas_per_sm)
-        with torch.cuda.device(self.device):
-            rc = self.lib.ncsb_create(ctypes.byref(self._handle), ctypes.byref(self.params))
+        # The handle's scratch comes from the caching allocator (three cudaMalloc
+        # and cudaFree calls took 1 ms of a short-lived solver); earlier work on
+        # the current stream may still use the block, so it is waited for.
+        with _on_device(self.device):
+            self._scratch = torch.empty(_lib.HANDLE_SCRATCH_BYTES, dtype=torch.uint8,
+                                        device=self.device)
+            torch.cuda.current_stream(self.device).synchronize()
+            rc = self.lib.ncsb_create_with_scratch(
+                ctypes.byref(self._handle), ctypes.byref(self.params), _ptr(self._scratch),
+                _lib.HANDLE_SCRATCH_BYTES)
         if rc != _lib.NCSB_OK:
             raise RuntimeError("ncsb_create failed with code %d" % rc)
         self.mask_shifted = None
@@ -171,12 +196,12 @@ class Solver:
             if tile_stats != "status":
                 cost = torch.empty(n, dtype=torch.float64, device=self.device)
                 evals = torch.empty(n, dtype=torch.int32, device=self.device)
-        s = launch_stream(stream, self.device, images, gamma, out, iters, status, cost, evals)
-        with torch.cuda.device(self.device):
+        s = launch_stream(stream, self.device, self._scratch, images, gamma, out, iters, status, cost, evals)
+        with _on_device(self.device):
             self._check(self.lib.ncsb_reduce_noise(
                 self._handle, _ptr(images), T, H, W, _ptr(gamma), per_frame, _ptr(out),
                 _ptr(iters), _ptr(status), _ptr(cost), _ptr(evals),
-                ctypes.c_void_p(s.cuda_stream)))
+                s.cuda_stream))
         if tile_stats == "all":
             return out, iters, status, cost, evals
         if tile_stats == "status":
@@ -215,13 +240,13 @@ class Solver:
             cost = torch.empty(n, dtype=torch.float64, device=self.device)
             evals = torch.empty(n, dtype=torch.int32, device=self.device)
         start = torch.empty(n, dtype=torch.int32, device=self.device)
-        s = launch_stream(stream, self.device, images, gamma, u0_tiles, out, iters, status, cost,
+        s = launch_stream(stream, self.device, self._scratch, images, gamma, u0_tiles, out, iters, status, cost,
                           evals, start)
-        with torch.cuda.device(self.device):
+        with _on_device(self.device):
             self._check(self.lib.ncsb_reduce_noise_start(
                 self._handle, _ptr(images), T, H, W, _ptr(gamma), per_frame, _ptr(u0_tiles),
                 _ptr(out), _ptr(iters), _ptr(status), _ptr(cost), _ptr(evals), _ptr(start),
-                ctypes.c_void_p(s.cuda_stream)))
+                s.cuda_stream))
         if not stats:
             return out, start
         return out, iters, status, cost, evals, start
@@ -278,12 +303,12 @@ class Solver:
             n = self.num_tiles(T, H, W)
             st = [torch.empty(n, dtype=torch.int32, device=self.device) for _ in range(3)]
             cost = torch.empty(n, dtype=torch.float64, device=self.device)
-        s = launch_stream(stream, self.device, adu, out, cost, *st, *keep)
-        with torch.cuda.device(self.device):
+        s = launch_stream(stream, self.device, self._scratch, adu, out, cost, *st, *keep)
+        with _on_device(self.device):
             self._check(self.lib.ncsb_reduce_noise_adu_typed(
                 self._handle, _ptr(adu), _ADU_TYPES[adu.dtype], T, H, W, ctypes.byref(cal),
                 _ptr(out), _ptr(st[0]), _ptr(st[1]), _ptr(cost), _ptr(st[2]),
-                ctypes.c_void_p(s.cuda_stream)))
+                s.cuda_stream))
         if tile_stats:
             return out, st[0], st[1], cost, st[2]
         return out
@@ -315,12 +340,12 @@ class Solver:
         elif (out.device.type != "cpu" or out.dtype != torch.float32
               or tuple(out.shape) != (T, H, W) or not out.is_contiguous()):
             raise ValueError("out must be a contiguous float32 host tensor [T, H, W]")
-        s = launch_stream(stream, self.device, *keep)
-        with torch.cuda.device(self.device):
+        s = launch_stream(stream, self.device, self._scratch, *keep)
+        with _on_device(self.device):
             self._check(self.lib.ncsb_reduce_noise_adu_host(
                 self._handle, _ptr(h_in), _ADU_TYPES[h_in.dtype], T, H, W, ctypes.byref(cal),
                 _ptr(out), int(chunk_frames or 0), int(n_streams or 0),
-                ctypes.c_void_p(s.cuda_stream)))
+                s.cuda_stream))
         return out
 
     # ---- batched launch: many stacks, each with its own alpha and mask ------
@@ -367,7 +392,7 @@ class Solver:
                 ctypes.memmove(a.mask_shifted, numpy.ascontiguousarray(ms).ctypes.data, 1024)
             keep.append((images, gamma, out))
             outs.append(out)
-        with torch.cuda.device(self.device):
+        with _on_device(self.device):
             self._check(self.lib.ncsb_batch_set(self._handle, arr, n))
         self._batch = keep
         n_tiles = ctypes.c_int64(0)
@@ -387,13 +412,13 @@ class Solver:
         if u0_tiles is not None:
             u0_tiles = self._tensor(u0_tiles, "u0_tiles", (self.batch_tiles, 16, 16))
         st = stats or {}
-        s = launch_stream(stream, self.device, u0_tiles, *st.values(),
+        s = launch_stream(stream, self.device, self._scratch, u0_tiles, *st.values(),
                           *[t for stack in self._batch for t in stack])
-        with torch.cuda.device(self.device):
+        with _on_device(self.device):
             self._check(self.lib.ncsb_batch_reduce_noise(
                 self._handle, _ptr(u0_tiles), _ptr(st.get("iters")), _ptr(st.get("status")),
                 _ptr(st.get("cost")), _ptr(st.get("evals")), _ptr(st.get("start")),
-                ctypes.c_void_p(s.cuda_stream)))
+                s.cuda_stream))
 
     def batch_stats(self):
         """Per-tile device tensors sized for the registered batch."""
@@ -443,11 +468,11 @@ class Solver:
         elif (out.device.type != "cpu" or out.dtype != torch.float32
               or tuple(out.shape) != (T, H, W) or not out.is_contiguous()):
             raise ValueError("out must be a contiguous float32 host tensor [T, H, W]")
-        s = launch_stream(stream, self.device)
-        with torch.cuda.device(self.device):
+        s = launch_stream(stream, self.device, self._scratch)
+        with _on_device(self.device):
             self._check(self.lib.ncsb_reduce_noise_host(
                 self._handle, _ptr(h_in), T, H, W, _ptr(h_g), per_frame, _ptr(out),
-                int(chunk_frames or 0), int(n_streams or 0), ctypes.c_void_p(s.cuda_stream)))
+                int(chunk_frames or 0), int(n_streams or 0), s.cuda_stream))
         return out
 
     def solve_tiles(self, data, gamma, u0=None, stream=None):
@@ -465,11 +490,11 @@ class Solver:
         status = torch.empty(n, dtype=torch.int32, device=self.device)
         cost = torch.empty(n, dtype=torch.float64, device=self.device)
         evals = torch.empty(n, dtype=torch.int32, device=self.device)
-        s = launch_stream(stream, self.device, data, gamma, u0, u, iters, status, cost, evals)
-        with torch.cuda.device(self.device):
+        s = launch_stream(stream, self.device, self._scratch, data, gamma, u0, u, iters, status, cost, evals)
+        with _on_device(self.device):
             self._check(self.lib.ncsb_solve_tiles(
                 self._handle, _ptr(data), _ptr(gamma), _ptr(u0), n, _ptr(u), _ptr(iters),
-                _ptr(status), _ptr(cost), _ptr(evals), ctypes.c_void_p(s.cuda_stream)))
+                _ptr(status), _ptr(cost), _ptr(evals), s.cuda_stream))
         self.last_evals = evals
         return u, iters, status, cost
 
@@ -563,16 +588,26 @@ class NCSCUDA:
             raise NCSCUDAException("gamma must have the same shape as the images!")
         solver = self._get_solver(alpha)
         solver.set_otf_mask_shifted(self.otf_mask)
-        host = torch.from_numpy(numpy.stack(images).astype(numpy.float32)).pin_memory()
-        ghost = torch.from_numpy(self.gamma).pin_memory()
         dev = solver.device
-        x = host.to(dev, non_blocking=True)
-        g = ghost.to(dev, non_blocking=True)
+        # one page-locked staging buffer both ways (from the caching host
+        # allocator), filled and emptied by torch's threaded copies
+        stage = torch.empty((len(images),) + im0_shape, dtype=torch.float32, pin_memory=True)
+        if all(im.dtype == numpy.float32 and im.flags.c_contiguous and im.flags.writeable
+               for im in images):
+            torch.stack([torch.from_numpy(im) for im in images], out=stage)
+        else:
+            stage.copy_(torch.from_numpy(numpy.stack(images).astype(numpy.float32)))
+        x = stage.to(dev, non_blocking=True)
+        g = torch.from_numpy(self.gamma).pin_memory().to(dev, non_blocking=True)
         out, iters, status = solver.reduce_noise(x, g, tile_stats="status")
-        result = out.cpu().numpy()
+        per_tile = torch.stack((status, iters)).to("cpu", non_blocking=True)
+        stage.copy_(out, non_blocking=True)
+        torch.cuda.current_stream(dev).synchronize()
+        result = stage.clone().numpy()
+        status, iters = per_tile.numpy()
         if verbose:
-            print("Processed {0:d} sub-regions.".format(iters.numel()))
-        _status_report(status.cpu().numpy(), iters.cpu().numpy(), verbose)
+            print("Processed {0:d} sub-regions.".format(iters.size))
+        _status_report(status, iters, verbose)
         return [result[i] for i in range(result.shape[0])]
 
 
@@ -645,7 +680,7 @@ def reduce_noise_normalized(images, gamma, mask3_centred, alpha=1.0, max_iters=1
         rc = lib.ncsb_reduce_noise_normalized(
             _ptr(images), T, H, W, _ptr(gamma), per_frame,
             m.ctypes.data_as(ctypes.POINTER(ctypes.c_float)), float(alpha), int(max_iters),
-            float(tol), _ptr(out), _ptr(it), _ptr(st), _ptr(cost), ctypes.c_void_p(s.cuda_stream))
+            float(tol), _ptr(out), _ptr(it), _ptr(st), _ptr(cost), s.cuda_stream)
     if rc != _lib.NCSB_OK:
         raise ValueError("ncsb_reduce_noise_normalized failed with code %d" % rc)
     if stats:
