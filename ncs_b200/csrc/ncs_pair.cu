@@ -17,12 +17,12 @@
 // a lane to share each row with three others.
 //
 // What bounds it (stack512, 200 x 512^2): instruction issue and FP32 time in
-// turn, 57 % of the issue slots and 45 % of the FMA pipe at 12 warps per SM, with
+// turn, 58 % of the issue slots and 46 % of the FMA pipe at 12 warps per SM, with
 // waits on fixed latencies and on instruction fetch between.  A pass takes 1,095
 // warp instructions for two tiles, where one tile per warp took 1,004 for one:
 // the lane's own transforms replace 47 % of those, and every reduction and
-// per-tile decision serves two tiles.  2.01 -> 1.34 ms (sensor2048: 15.73 ->
-// 10.48 ms).  Two tiles of a pair rarely differ in iterations (5.04 each, 5.09
+// per-tile decision serves two tiles.  2.01 -> 1.31 ms (sensor2048: 15.75 ->
+// 10.22 ms).  Two tiles of a pair rarely differ in iterations (5.04 each, 5.09
 // for the slower of two), so they run in lock step and a half that ends first
 // idles.
 #include "ncs_warp_common.cuh"
@@ -257,6 +257,7 @@ ncs_pair_kernel(const SolveArgs a, const int one_wave) {
                        kr * kTabRow;
     bool asym = false;  // any bin with M^2(kr, kc) != M^2(kr, -kc)
     float alpha = a.alpha;
+    long long st_begin = 0, st_end = 0;  // Batch: tiles of the half's current stack
     if constexpr (!Batch) {
         float* ct = reinterpret_cast<float*>(dsm);
         bool diff = false;
@@ -287,31 +288,37 @@ ncs_pair_kernel(const SolveArgs a, const int one_wave) {
         bool act = 2 * pair + h < a.n_tiles;
         long long lt = tile;  // index of the tile within its stack
         if constexpr (Batch) {
-            int lo = 0, hi = a.n_stacks - 1;
-            while (lo < hi) {  // last stack whose first tile is <= tile
-                const int mid = (lo + hi + 1) >> 1;
-                if (__ldg(&a.stacks[mid].tile_begin) <= tile) lo = mid;
-                else hi = mid - 1;
-            }
-            __syncwarp();
-            if (c == 0) sdesc[h] = a.stacks[lo];
-            // the half's weight tables from the stack's lane-layout table
-            const float* ml = a.mk_lane + (size_t)lo * 256;
-            bool diff = false;
-            for (int idx = c; idx < kTab; idx += 16) {
-                const int r = idx / kTabRow, k = idx - r * kTabRow;
-                if (k < 9) {
-                    const int kn = (16 - k) & 15, i = bitrev3(r >> 1);
-                    const float s = tab_scale(r, k);
-                    const float A = __ldg(ml + (2 * k + (r & 1)) * 8 + i);
-                    const float B = __ldg(ml + (2 * kn + (r & 1)) * 8 + i);
-                    btab[h * kTabFloats + idx] = s * A;
-                    btab[h * kTabFloats + kTab + idx] = s * B;
-                    diff = diff || A != B;
+            // the half's stack, when this tile is not in the last one's (looking it
+            // up for every tile cost 5 %: 16 stacks, 0.66 -> 0.62 ms)
+            if (__any_sync(kFull, tile < st_begin || tile >= st_end)) {
+                int lo = 0, hi = a.n_stacks - 1;
+                while (lo < hi) {  // last stack whose first tile is <= tile
+                    const int mid = (lo + hi + 1) >> 1;
+                    if (__ldg(&a.stacks[mid].tile_begin) <= tile) lo = mid;
+                    else hi = mid - 1;
                 }
+                st_begin = __ldg(&a.stacks[lo].tile_begin);
+                st_end = lo + 1 < a.n_stacks ? __ldg(&a.stacks[lo + 1].tile_begin) : a.n_tiles;
+                __syncwarp();
+                if (c == 0) sdesc[h] = a.stacks[lo];
+                // the half's weight tables from the stack's lane-layout table
+                const float* ml = a.mk_lane + (size_t)lo * 256;
+                bool diff = false;
+                for (int idx = c; idx < kTab; idx += 16) {
+                    const int r = idx / kTabRow, k = idx - r * kTabRow;
+                    if (k < 9) {
+                        const int kn = (16 - k) & 15, i = bitrev3(r >> 1);
+                        const float s = tab_scale(r, k);
+                        const float A = __ldg(ml + (2 * k + (r & 1)) * 8 + i);
+                        const float B = __ldg(ml + (2 * kn + (r & 1)) * 8 + i);
+                        btab[h * kTabFloats + idx] = s * A;
+                        btab[h * kTabFloats + kTab + idx] = s * B;
+                        diff = diff || A != B;
+                    }
+                }
+                asym = __any_sync(kFull, diff);
+                __syncwarp();
             }
-            asym = __any_sync(kFull, diff);
-            __syncwarp();
             lt = tile - sdesc[h].tile_begin;
             alpha = sdesc[h].alpha;
         }
@@ -866,21 +873,47 @@ ncs_pair_kernel(const SolveArgs a, const int one_wave) {
             // ---- outputs of the halves that ended with this pass ---------------------
             if (__any_sync(kFull, fin)) {
                 if (a.cost) {
-                    float2 nc[8], gm[8];
-                    load_vec(terms, lane, nc);
-                    load_vec(gterm, lane, gm);
-                    double e0 = 0.0, e1 = 0.0;
+                    if constexpr (Batch) {
+                        float2 nc[8], gm[8];
+                        load_vec(terms, lane, nc);
+                        load_vec(gterm, lane, gm);
+                        double e0 = 0.0, e1 = 0.0;
 #pragma unroll
-                    for (int j = 0; j < 8; ++j)
+                        for (int j = 0; j < 8; ++j)
 #pragma unroll
-                        for (int e = 0; e < 2; ++e) {
-                            const double ui = e ? u[j].y : u[j].x, gi = e ? gm[j].y : gm[j].x;
-                            e0 += ui + (double)(e ? nc[j].y : nc[j].x) * log(fmax(ui + gi, 1.0e-6));
-                            e1 += ui * (e ? v[j].y : v[j].x);
+                            for (int e = 0; e < 2; ++e) {
+                                const double ui = e ? u[j].y : u[j].x, gi = e ? gm[j].y : gm[j].x;
+                                e0 += ui + (double)(e ? nc[j].y : nc[j].x) * log(fmax(ui + gi, 1.0e-6));
+                                e1 += ui * (e ? v[j].y : v[j].x);
+                            }
+                        e0 = half_sum_d(e0);
+                        e1 = half_sum_d(e1);
+                        if (fin && c == 0) a.cost[tile] = e0 + 0.5 * e1;  // v = 2 alpha Q u
+                    } else {
+                        // rolled, with u through shared memory: sixteen inlined FP64 logs
+                        // are as much code as the pass and cost the instruction cache
+                        // 2.5 % of a solve that does not ask for them (the batched
+                        // instance ran 6 % slower rolled)
+                        double e0 = 0.0, e1 = 0.0;
+                        __syncwarp();
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) {
+                            buf[(2 * j) * kRow + c] = u[j].x;
+                            buf[(2 * j + 1) * kRow + c] = u[j].y;
+                            e1 += (double)u[j].x * v[j].x;
+                            e1 += (double)u[j].y * v[j].y;
                         }
-                    e0 = half_sum_d(e0);
-                    e1 = half_sum_d(e1);
-                    if (fin && c == 0) a.cost[tile] = e0 + 0.5 * e1;  // v = 2 alpha Q u
+#pragma unroll 1
+                        for (int r = 0; r < 16; ++r) {
+                            const int at = (r >> 2) * 128 + lane * 4 + (r & 3);
+                            const double ui = buf[r * kRow + c];
+                            e0 += ui + (double)reinterpret_cast<const float*>(terms)[at] *
+                                           log(fmax(ui + reinterpret_cast<const float*>(gterm)[at], 1.0e-6));
+                        }
+                        e0 = half_sum_d(e0);
+                        e1 = half_sum_d(e1);
+                        if (fin && c == 0) a.cost[tile] = e0 + 0.5 * e1;  // v = 2 alpha Q u
+                    }
                 }
                 if (fin) {
                     act = false;
