@@ -47,6 +47,12 @@ def test_result_does_not_depend_on_the_partner(cuda_ok, n, mask):
     assert int(st2[0]) != 0
     for a, b in ((u, u2), (it, it2), (st, st2), (cost, cost2)):
         assert torch.equal(a, b[1:].flip(0))
+    if mask == "random":
+        # these masks weight the mean (M(0) = 1), which the bright tiles' cost cannot
+        # follow within the cap: a quarter of the tiles end there in every solver
+        # form, so there is no optimum to compare with (random masks on ordinary
+        # tiles: test_gpu_plain.py, test_gpu_batch.py)
+        return
     # the optimum (cost gap 1e-6 relative, as the parity tests of the other forms)
     k = min(n, 48)
     un = u[:k].cpu().numpy().astype(numpy.float64)
