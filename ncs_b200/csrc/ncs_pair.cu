@@ -370,15 +370,20 @@ ncs_pair_kernel(const SolveArgs a, const int one_wave) {
             // no pair yet: a zero history with rho = 0 leaves every update out
 #pragma unroll
             for (int j = 0; j < 8; ++j) nc[j] = make_float2(0.0f, 0.0f);
-            store_vec(hs, lane, nc);
             store_vec(hy, lane, nc);
             store_vec(hq, lane, nc);
-            if (Warm) {
+            if constexpr (Warm) {
+                // s's place first holds u0 - d, for the start pass
                 const float* ut = a.u0 + tile * kPix + c;
 #pragma unroll
-                for (int r = 0; r < 16; ++r)
-                    (r & 1 ? u[r >> 1].y : u[r >> 1].x) = __ldg(ut + r * kTile);
+                for (int r = 0; r < 16; ++r) {
+                    float& ui = r & 1 ? u[r >> 1].y : u[r >> 1].x;
+                    const float di = ui;
+                    ui = __ldg(ut + r * kTile);
+                    (r & 1 ? nc[r >> 1].y : nc[r >> 1].x) = __fsub_rn(ui, di);
+                }
             }
+            store_vec(hs, lane, nc);
         }
 
         // ---- preconditioned L-BFGS, both tiles in lock step -----------------------
@@ -516,8 +521,8 @@ ncs_pair_kernel(const SolveArgs a, const int one_wave) {
                 if (Warm && start_pass == 2) {
                     // the bound of ncs_spectral.cu: accept a proposal with
                     // LL(u0) - LL(d) + (u0 - d)'v0 <= 0 without transforming d
-                    float2 dd[8], nc[8], gm[8];
-                    load_tile(dd, nullptr);
+                    float2 de[8], nc[8], gm[8];
+                    load_vec(hs, lane, de);
                     load_vec(terms, lane, nc);
                     load_vec(gterm, lane, gm);
                     double bound = 0.0;
@@ -528,13 +533,13 @@ ncs_pair_kernel(const SolveArgs a, const int one_wave) {
                         for (int j = 4 * b; j < 4 * b + 4; ++j)
 #pragma unroll
                             for (int e = 0; e < 2; ++e) {
-                                const float ui = e ? u[j].y : u[j].x, di = e ? dd[j].y : dd[j].x;
+                                const float ui = e ? u[j].y : u[j].x, di = e ? de[j].y : de[j].x;
                                 const float gi = e ? gm[j].y : gm[j].x, ci = e ? nc[j].y : nc[j].x;
                                 const float pi = e ? p[j].y : p[j].x;
                                 const float lr = __fsub_rn(__logf(fmaxf(ui + gi, kFitMin)),
-                                                           __logf(fmaxf(di + gi, kFitMin)));
-                                dl += fmaf(ci, lr, ui - di);
-                                dq += __fmul_rn(__fsub_rn(ui, di), pi);
+                                                           __logf(fmaxf(-ci, kFitMin)));
+                                dl += fmaf(ci, lr, di);
+                                dq += __fmul_rn(di, pi);
                             }
                         bound += (double)dl + (double)dq;
                     }
@@ -580,6 +585,12 @@ ncs_pair_kernel(const SolveArgs a, const int one_wave) {
 #pragma unroll
                         for (int j = 0; j < 8; ++j) u[j] = dd[j];
                     }
+                }
+                if constexpr (Warm) {
+                    float2 z[8];
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) z[j] = make_float2(0.0f, 0.0f);
+                    store_vec(hs, lane, z);
                 }
                 start_pass = 0;
                 first = false;
