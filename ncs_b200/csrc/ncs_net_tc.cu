@@ -421,14 +421,26 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
 // y = acc * scale + bias.  E4M3: the accumulator carries the input and
 // weight scales, the stored activation the next layer's input scale (a
 // positive factor, so it commutes with the ReLU).  All threads of the CTA
-// take part; inv_wscale (128 floats, shared) is scratch.  Ends with
-// __syncthreads.
+// take part; inv_wscale (128 floats, shared) and stage (kNetParams floats,
+// shared) are scratch.  Ends with __syncthreads.
+//
+// The parameters are staged in shared memory by one coalesced pass and the
+// column maxima shared out over the warps: reading them from global memory where
+// they are used, 128 threads in serial chains of 288, took 100 us of every launch
+// (50 x 512^2 proposals and their solve 1.39 -> 1.29 ms, one small frame 99 ->
+// 44 us).
+constexpr int kNetParams = 2 * 9 * kC + kC + 2 * (kC * 9 * kC + kC) + kC * 9 + 1;
 template <bool F8>
 __device__ void load_network(const float* __restrict__ params, unsigned char* sW1,
                              unsigned char* sW2, unsigned char* sW3, int tap_bytes,
                              unsigned char* sW4, float* sScale, float* sBias, float* inv_wscale,
-                             int t, int nthr, bool w4_per_tap = false) {
-    const float* w1 = params;
+                             int t, int nthr, float* stage, bool w4_per_tap = false) {
+#pragma unroll 8
+    for (int i = t; i < kNetParams; i += nthr) stage[i] = params[i];
+    int* mx = reinterpret_cast<int*>(inv_wscale);  // |w| >= 0: ordered as its bits
+    for (int i = t; i < 4 * kC; i += nthr) mx[i] = 0;
+    __syncthreads();
+    const float* w1 = stage;
     const float* b1 = w1 + 2 * 9 * kC;
     const float* w2 = b1 + kC;
     const float* b2 = w2 + kC * 9 * kC;
@@ -442,13 +454,22 @@ __device__ void load_network(const float* __restrict__ params, unsigned char* sW
         if (l == 3) return co == 0 ? w4[ci * 9 + tap] : 0.0f;
         return (l == 1 ? w2 : w3)[(ci * 9 + tap) * kC + co];
     };
-    if (t < 4 * kC) {  // thread t: output column co = t & 31 of layer l = t >> 5
-        const int l = t >> 5, co = t & 31, cin = l == 0 ? 2 : kC;
-        float mx = 0.0f;
-        if (F8)
-            for (int ci = 0; ci < cin; ++ci)
-                for (int tap = 0; tap < 9; ++tap) mx = fmaxf(mx, fabsf(weight(l, ci, tap, co)));
-        inv_wscale[t] = mx > 0.0f ? kF8Max / mx : 1.0f;
+    if (F8) {  // column maxima: 96 columns in parts of the input channels, and w4
+        const int parts = nthr / 96, col = t % 96, l = col >> 5, co = col & 31;
+        float m = 0.0f;
+        if (t < 96 * parts)
+            for (int ci = t / 96; ci < (l == 0 ? 2 : kC); ci += parts)
+#pragma unroll
+                for (int tap = 0; tap < 9; ++tap) m = fmaxf(m, fabsf(weight(l, ci, tap, co)));
+        if (t < 96 * parts) atomicMax(mx + col, __float_as_int(m));
+        m = 0.0f;
+        for (int i = t; i < kC * 9; i += nthr) m = fmaxf(m, fabsf(w4[i]));
+        if (t < kC * 9) atomicMax(mx + 96, __float_as_int(m));
+        __syncthreads();
+    }
+    if (t < 4 * kC) {  // column co = t & 31 of layer t >> 5
+        const float m = __int_as_float(mx[t]);
+        inv_wscale[t] = m > 0.0f ? kF8Max / m : 1.0f;
     }
     __syncthreads();
     for (int i = t; i < 32 * 32; i += nthr) {
@@ -541,6 +562,7 @@ __global__ void __launch_bounds__(kCtaThreads)
     infer_tc(const Src src, const float* __restrict__ params, float* __restrict__ u0,
              int32_t* __restrict__ status) {
     using F = Fmt<F8>;
+    static_assert(kSlots * F::kActBytes >= kNetParams * 4, "parameter staging");
     extern __shared__ __align__(1024) unsigned char sm[];
     __shared__ __align__(8) uint64_t full_bar[kSlots];   // a slot's layer MMAs completed
     __shared__ __align__(8) uint64_t ready_bar[kSlots];  // a slot's next operand written
@@ -556,7 +578,8 @@ __global__ void __launch_bounds__(kCtaThreads)
     float* sScale = reinterpret_cast<float*>(sm + F::kOffScale);
     float* sBias = reinterpret_cast<float*>(sm + F::kOffBias);
     load_network<F8>(params, sm + F::kOffW1, sm + F::kOffW2, sm + F::kOffW3, F::kWtapBytes,
-                     sm + F::kOffW4, sScale, sBias, inv_wscale, t, nthr);
+                     sm + F::kOffW4, sScale, sBias, inv_wscale, t, nthr,
+                     reinterpret_cast<float*>(sm + F::kOffAct));
     for (int i = t; i < kEpiGroups * kStageBytes / 16; i += nthr)  // rows never written stay 0
         reinterpret_cast<uint4*>(sm + F::kOffStage)[i] = make_uint4(0u, 0u, 0u, 0u);
     for (int i = t; i < kSlots * kTileBytes / 16; i += nthr)  // the feature planes' border
@@ -972,6 +995,7 @@ __global__ void __launch_bounds__(w16::kThreadsW)
     infer_tc_w16(const Src src, const float* __restrict__ params, float* __restrict__ u0,
                  int32_t* __restrict__ status) {
     using namespace w16;
+    static_assert(kSlotsW * kSlotBytes >= kNetParams * 4, "parameter staging");
     extern __shared__ __align__(1024) unsigned char sm[];
     __shared__ __align__(8) uint64_t full_bar[kSlotsW];   // a slot's layer MMAs completed
     __shared__ __align__(8) uint64_t ready_bar[kSlotsW];  // a slot's next operand written
@@ -985,7 +1009,8 @@ __global__ void __launch_bounds__(w16::kThreadsW)
     float* sScale = reinterpret_cast<float*>(sm + kOffScale);
     float* sBias = reinterpret_cast<float*>(sm + kOffBias);
     load_network<true>(params, sm + kOffW1, sm + kOffW2, sm + kOffW3, kWtapBytes, sm + kOffW4,
-                       sScale, sBias, inv_wscale, t, nthr, true);
+                       sScale, sBias, inv_wscale, t, nthr, reinterpret_cast<float*>(sm + kOffCopies),
+                       true);
     // the copies (their zero rows and columns are never written) and the
     // feature planes' border
     for (int i = t; i < kSlotsW * kSlotBytes / 16; i += nthr)
