@@ -49,65 +49,83 @@ __device__ __forceinline__ float clamp_d(float dv) { return dv <= 0.0f ? 1.0e-6f
 // of once per frame.
 constexpr int kFramesPerThread = 8;
 
-// Grid: x over groups of 4 pixels of a frame, y over chunks of
-// kFramesPerThread frames (y-stride past 65535 chunks).  vec (set by the
-// host: one map pair, a frame size divisible by 4 and every pointer aligned
-// for it): 4-wide loads and 16-byte stores.  gamma_frames: [T][H][W] with
-// several pairs (gamma depends on the level), else null; gamma_map: [H][W],
-// written by the threads of frame 0, or null.
+// Four pixels a thread (one map pair, a frame size divisible by 4 and every
+// pointer aligned for it): 4-wide loads and 16-byte stores.  Grid: x over groups
+// of 4 pixels, y over chunks of kFramesPerThread frames (y-stride past 65535
+// chunks).  gamma_map: [H][W], written by the threads of frame 0, or null.
 template <typename In>
-__global__ void __launch_bounds__(256) convert(const In* __restrict__ adu, int T, long long hw,
-                                               const float* __restrict__ offset,
-                                               const float* __restrict__ gain,
-                                               const float* __restrict__ var, int n_levels,
-                                               float l0, float l1, float l2, int vec,
-                                               float* __restrict__ d,
-                                               float* __restrict__ gamma_frames,
-                                               float* __restrict__ gamma_map) {
-    const long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;  // pixel group
-    const long long p0 = 4 * q;
+__global__ void __launch_bounds__(256) convert4(const In* __restrict__ adu, int T, long long hw,
+                                                const float* __restrict__ offset,
+                                                const float* __restrict__ gain,
+                                                const float* __restrict__ var,
+                                                float* __restrict__ d,
+                                                float* __restrict__ gamma_map) {
+    const long long p0 = 4 * ((long long)blockIdx.x * blockDim.x + threadIdx.x);
     if (p0 >= hw) return;
-    if (vec) {
-        const float4 off = __ldg(reinterpret_cast<const float4*>(offset + p0));
-        const float4 gn = __ldg(reinterpret_cast<const float4*>(gain + p0));
-        if (blockIdx.y == 0 && gamma_map) {
-            const float4 vv = __ldg(reinterpret_cast<const float4*>(var + p0));
-            *reinterpret_cast<float4*>(gamma_map + p0) =
-                make_float4(vv.x / (gn.x * gn.x), vv.y / (gn.y * gn.y), vv.z / (gn.z * gn.z),
-                            vv.w / (gn.w * gn.w));
-        }
-        for (long long t0 = (long long)blockIdx.y * kFramesPerThread; t0 < T;
-             t0 += (long long)gridDim.y * kFramesPerThread) {
-            const int n = T - t0 < kFramesPerThread ? (int)(T - t0) : kFramesPerThread;
-#pragma unroll 4
-            for (int k = 0; k < n; ++k) {
-                const long long i0 = (t0 + k) * hw + p0;
-                const float4 av = load4(adu + i0);
-                *reinterpret_cast<float4*>(d + i0) = make_float4(
-                    clamp_d((av.x - off.x) / gn.x), clamp_d((av.y - off.y) / gn.y),
-                    clamp_d((av.z - off.z) / gn.z), clamp_d((av.w - off.w) / gn.w));
-            }
-        }
-        return;
+    const float4 off = __ldg(reinterpret_cast<const float4*>(offset + p0));
+    const float4 gn = __ldg(reinterpret_cast<const float4*>(gain + p0));
+    if (blockIdx.y == 0 && gamma_map) {
+        const float4 vv = __ldg(reinterpret_cast<const float4*>(var + p0));
+        *reinterpret_cast<float4*>(gamma_map + p0) =
+            make_float4(vv.x / (gn.x * gn.x), vv.y / (gn.y * gn.y), vv.z / (gn.z * gn.z),
+                        vv.w / (gn.w * gn.w));
     }
     for (long long t0 = (long long)blockIdx.y * kFramesPerThread; t0 < T;
          t0 += (long long)gridDim.y * kFramesPerThread) {
-        const long long t1 = T - t0 < kFramesPerThread ? T : t0 + kFramesPerThread;
-        for (long long t = t0; t < t1; ++t) {
-            for (long long p = p0; p < p0 + 4 && p < hw; ++p) {
-                const long long i = t * hw + p;
-                const float av = load1(adu + i);
-                // the pair of the pixel's ADU level: level k for levels[k-1] <= ADU
-                int lv = 0;
-                lv += (1 < n_levels && av >= l0) ? 1 : 0;
-                lv += (2 < n_levels && av >= l1) ? 1 : 0;
-                lv += (3 < n_levels && av >= l2) ? 1 : 0;
-                const long long at = (long long)lv * hw + p;
-                const float gn = __ldg(gain + at);
-                d[i] = clamp_d((av - __ldg(offset + p)) / gn);
-                if (gamma_frames) gamma_frames[i] = __ldg(var + at) / (gn * gn);
-                if (t == 0 && gamma_map) gamma_map[p] = __ldg(var + p) / (gn * gn);
-            }
+        const int n = T - t0 < kFramesPerThread ? (int)(T - t0) : kFramesPerThread;
+#pragma unroll 4
+        for (int k = 0; k < n; ++k) {
+            const long long i0 = (t0 + k) * hw + p0;
+            const float4 av = load4(adu + i0);
+            *reinterpret_cast<float4*>(d + i0) = make_float4(
+                clamp_d((av.x - off.x) / gn.x), clamp_d((av.y - off.y) / gn.y),
+                clamp_d((av.z - off.z) / gn.z), clamp_d((av.w - off.w) / gn.w));
+        }
+    }
+}
+
+// One pixel a thread: any frame size, alignment and number of map pairs L.  A
+// warp's accesses are consecutive, and the pixel's L gains and gammas stay in
+// registers for the chunk.  (Four consecutive pixels a thread, one after the
+// other, reloaded the maps for every frame: 60 16-bit frames of 411 x 301 took 28
+// us, now 19; 8-bit with three pairs 40, now 27.)  gamma_frames: [T][H][W] with
+// several pairs (gamma depends on the level), else null.
+template <typename In, int L>
+__global__ void __launch_bounds__(256) convert1(const In* __restrict__ adu, int T, long long hw,
+                                                const float* __restrict__ offset,
+                                                const float* __restrict__ gain,
+                                                const float* __restrict__ var, float l0, float l1,
+                                                float l2, float* __restrict__ d,
+                                                float* __restrict__ gamma_frames,
+                                                float* __restrict__ gamma_map) {
+    const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= hw) return;
+    const float off = __ldg(offset + p);
+    float gn[L], gm[L];
+#pragma unroll
+    for (int q = 0; q < L; ++q) {
+        gn[q] = __ldg(gain + q * hw + p);
+        gm[q] = __ldg(var + q * hw + p) / (gn[q] * gn[q]);
+    }
+    if (blockIdx.y == 0 && gamma_map) gamma_map[p] = gm[0];
+    const float lev[3] = {l0, l1, l2};
+    for (long long t0 = (long long)blockIdx.y * kFramesPerThread; t0 < T;
+         t0 += (long long)gridDim.y * kFramesPerThread) {
+        const int n = T - t0 < kFramesPerThread ? (int)(T - t0) : kFramesPerThread;
+#pragma unroll 4
+        for (int k = 0; k < n; ++k) {
+            const long long i = (t0 + k) * hw + p;
+            const float av = load1(adu + i);
+            // the pair of the pixel's ADU level: pair q from levels[q-1] on (ascending)
+            float g = gn[0], m = gm[0];
+#pragma unroll
+            for (int q = 1; q < L; ++q)
+                if (av >= lev[q - 1]) {
+                    g = gn[q];
+                    m = gm[q];
+                }
+            d[i] = clamp_d((av - off) / g);
+            if (gamma_frames) gamma_frames[i] = m;
         }
     }
 }
@@ -132,12 +150,20 @@ cudaError_t launch_typed(const In* adu, int T, long long hw, const ncsb_calibrat
     const bool vec = cal->n_levels == 1 && hw % 4 == 0 && aligned(adu, 4 * sizeof(In)) &&
                      aligned(cal->offset, 16) && aligned(cal->gain, 16) &&
                      aligned(cal->variance, 16) && aligned(d, 16) && aligned(gamma_map, 16);
-    const long long groups = (hw + 3) / 4;
     const long long chunks = (T + kFramesPerThread - 1) / kFramesPerThread;
-    const dim3 grid((unsigned)((groups + 255) / 256), (unsigned)(chunks < 65535 ? chunks : 65535));
-    convert<In><<<grid, 256, 0, s>>>(adu, T, hw, cal->offset, cal->gain, cal->variance,
-                                     cal->n_levels, cal->levels[0], cal->levels[1],
-                                     cal->levels[2], vec ? 1 : 0, d, gamma_frames, gamma_map);
+    const long long px = vec ? hw / 4 : hw;
+    const dim3 grid((unsigned)((px + 255) / 256), (unsigned)(chunks < 65535 ? chunks : 65535));
+    if (vec) {
+        convert4<In><<<grid, 256, 0, s>>>(adu, T, hw, cal->offset, cal->gain, cal->variance, d,
+                                          gamma_map);
+        return cudaGetLastError();
+    }
+    const auto kernel = cal->n_levels == 1   ? convert1<In, 1>
+                        : cal->n_levels == 2 ? convert1<In, 2>
+                        : cal->n_levels == 3 ? convert1<In, 3>
+                                             : convert1<In, 4>;
+    kernel<<<grid, 256, 0, s>>>(adu, T, hw, cal->offset, cal->gain, cal->variance, cal->levels[0],
+                                cal->levels[1], cal->levels[2], d, gamma_frames, gamma_map);
     return cudaGetLastError();
 }
 
