@@ -230,7 +230,13 @@ __device__ constexpr float kFarPoly[9] = {2.0f,         0.666660494f, 0.40032141
 // share the queue; each half finds its tile's stack by binary search.
 // `one_wave`: the grid holds a warp for every pair of tiles, so warps take
 // their pair by index and the queue is not touched.
-template <int MinBlocks, bool Warm, bool Batch>
+// Late: a warp takes its first pair by index and, for the last two pairs that
+// it can expect, draws the next one only when it is free: a pair drawn ahead
+// waits for whoever drew it, and just above a full wave that doubled the
+// launch (848 x 848, 3,721 tiles: 39.7 -> 30.4 us; 3.7 waves: 77.0 -> 75.7).
+// Elsewhere the draw's latency hides behind the solve.  A batch draws late
+// throughout (16 stacks: 627 -> 580 us; with the far draws ahead 597).
+template <int MinBlocks, bool Warm, bool Batch, bool Late>
 __global__ void __launch_bounds__(kWarpCtaThreads, MinBlocks)
 ncs_pair_kernel(const SolveArgs a, const int one_wave) {
     extern __shared__ __align__(16) unsigned char dsm[];
@@ -275,15 +281,17 @@ ncs_pair_kernel(const SolveArgs a, const int one_wave) {
     }
 
     long long pair = (long long)wid * gridDim.x + blockIdx.x;
-    if (!one_wave) {
+    if (!Late && !one_wave) {
         unsigned long long tk = 0;
         if (lane == 0) tk = atomicAdd(a.queue, 1ull);
         pair = (long long)__shfl_sync(kFull, tk, 0);
     }
+    const long long late_from = n_pairs - 8LL * gridDim.x;
     while (pair < n_pairs) {
         // the next pair's index, fetched while this one is solved
         unsigned long long tk = 0;
-        if (!one_wave && lane == 0) tk = atomicAdd(a.queue, 1ull);
+        const bool ahead = Late ? !Batch && pair < late_from : !one_wave;
+        if (ahead && lane == 0) tk = atomicAdd(a.queue, 1ull);
         const long long tile = min(2 * pair + h, a.n_tiles - 1);
         bool act = 2 * pair + h < a.n_tiles;
         long long lt = tile;  // index of the tile within its stack
@@ -952,8 +960,14 @@ ncs_pair_kernel(const SolveArgs a, const int one_wave) {
                 if (!__any_sync(kFull, act)) break;
             }
         }
-        if (one_wave) pair += 4LL * gridDim.x;
-        else pair = (long long)__shfl_sync(kFull, tk, 0);
+        if constexpr (Late) {
+            if (one_wave) break;
+            if (!ahead && lane == 0) tk = atomicAdd(a.queue, 1ull);
+            pair = (long long)__shfl_sync(kFull, tk, 0) + 4LL * gridDim.x;
+        } else {
+            if (one_wave) pair += 4LL * gridDim.x;
+            else pair = (long long)__shfl_sync(kFull, tk, 0);
+        }
         __syncwarp();  // every lane is done with this pair's shared memory
     }
 }
@@ -967,11 +981,18 @@ constexpr int kPairBlocks = 3;
 
 using PairFn = void (*)(SolveArgs, int);
 
-PairFn pair_variant(bool warm, bool batch) {
-    if (batch) return warm ? ncs_pair_kernel<kPairBlocks, true, true>
-                           : ncs_pair_kernel<kPairBlocks, false, true>;
-    return warm ? ncs_pair_kernel<kPairBlocks, true, false>
-                : ncs_pair_kernel<kPairBlocks, false, false>;
+// Launches of this many waves draw ahead to the end: the tail is short there
+// and the plainer loop compiles to the faster pass (stack512, 7.7 waves:
+// 1,306 us against 1,326).  Launches with proposals gained at every size
+// (512 frames of 512 x 512: 1,287 -> 1,279 us).
+constexpr long long kAheadWaves = 4;
+
+PairFn pair_variant(bool warm, bool batch, bool late) {
+    if (batch) return warm ? ncs_pair_kernel<kPairBlocks, true, true, true>
+                           : ncs_pair_kernel<kPairBlocks, false, true, true>;
+    if (warm) return ncs_pair_kernel<kPairBlocks, true, false, true>;
+    return late ? ncs_pair_kernel<kPairBlocks, false, false, true>
+                : ncs_pair_kernel<kPairBlocks, false, false, false>;
 }
 
 }  // namespace
@@ -993,17 +1014,23 @@ bool pair_one_wave(long long n_tiles, int ctas_per_sm, int num_sms) {
 // Resolves a variant's attributes (before a stream capture, say).
 cudaError_t pair_prepare(bool warm, bool batch) {
     const size_t smem = batch ? pair_smem_bytes<true>() : pair_smem_bytes<false>();
-    return cudaFuncSetAttribute(pair_variant(warm, batch),
-                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    for (const bool late : {false, true}) {
+        const cudaError_t e = cudaFuncSetAttribute(pair_variant(warm, batch, late),
+                                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                   (int)smem);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
 }
 
 cudaError_t launch_pair(const SolveArgs& args, int ctas_per_sm, int num_sms, cudaStream_t stream) {
     const bool warm = args.u0 != nullptr, batch = args.stacks != nullptr;
-    const PairFn fn = pair_variant(warm, batch);
-    const size_t smem = batch ? pair_smem_bytes<true>() : pair_smem_bytes<false>();
-    cudaError_t e = pair_prepare(warm, batch);
-    if (e != cudaSuccess) return e;
     const long long grid = pair_grid(args.n_tiles, ctas_per_sm, num_sms);
+    const PairFn fn = pair_variant(warm, batch, (args.n_tiles + 1) / 2 < kAheadWaves * 4 * grid);
+    const size_t smem = batch ? pair_smem_bytes<true>() : pair_smem_bytes<false>();
+    const cudaError_t e =
+        cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
     fn<<<(unsigned)grid, kWarpCtaThreads, smem, stream>>>(
         args, pair_one_wave(args.n_tiles, ctas_per_sm, num_sms) ? 1 : 0);
     return cudaGetLastError();

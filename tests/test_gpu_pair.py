@@ -61,3 +61,28 @@ def test_result_does_not_depend_on_the_partner(cuda_ok, n, mask):
     best = best[0] if isinstance(best, tuple) else best
     gap = nr.rel_cost_gap(nr.cost(un, dk, gk, ms, 0.2), nr.cost(best, dk, gk, ms, 0.2))
     assert numpy.max(gap) < 1e-6
+
+
+@pytest.mark.parametrize("ctas", [1, 0])
+@pytest.mark.parametrize("more", [-24, -1, 0, 3])
+def test_every_tile_is_solved_once_around_the_change_of_draw(cuda_ok, more, ctas):
+    """Launches just below, at and above four pairs per warp, where the kernel
+    changes when it draws its next pair: each tile's result is that of a small
+    launch (with all proposals off and on), whatever warp took it."""
+    import ncs_b200
+    rng = numpy.random.default_rng(5)
+    d, g = (torch.from_numpy(x).cuda() for x in tiles(64, rng))
+    per = ctas if ctas else 3
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    n = 2 * 4 * 4 * per * sms + more
+    s = ncs_b200.Solver(alpha=0.2, epsilon=1e-6, max_iters=40, ctas_per_sm=ctas)
+    s.set_otf_mask_shifted(create_otf_mask_shifted())
+    at = torch.arange(n, device="cuda") % 64
+    for u0 in (None, d * 0.9 + 1.0):
+        kw = {} if u0 is None else {"u0": u0}
+        kwn = {} if u0 is None else {"u0": u0[at].contiguous()}
+        small = s.solve_tiles(d, g, **kw)
+        big = s.solve_tiles(d[at].contiguous(), g[at].contiguous(), **kwn)
+        for a, b in zip(small, big):
+            if a is not None:
+                assert torch.equal(a[at], b)
