@@ -67,15 +67,15 @@ for _f in ("tc_tf32", "tc_bf16x3"):
 # kernel on stack512 at 64 frames, at the commit named in WARP_INST_MEASURED.
 # Used for the issue-rate bound, the one that limits these kernels; a kernel
 # changed since that commit needs a new capture.
-WARP_INST_PER_PASS = {"spectral": 532251760 / (87616 * 6.047982),
+WARP_INST_PER_PASS = {"spectral": 290407027 / (87616 * 6.047982),
                       "plain": 2130097923 / (87616 * 15.693230),
                       "plain_wg": 7479161369 / (87616 * 15.5538)}
 # multiply-adds x 2 of the warm-start network per 16x16 tile:
 # 256 px x 9 taps x (2*32 + 32*32 + 32*32 + 32*1)
 INFER_FLOP_PER_TILE = 2 * 256 * 9 * (2 * 32 + 32 * 32 + 32 * 32 + 32 * 1)
-WARP_INST_MEASURED = {"spectral": "35be777", "plain": "3d152ab", "plain_wg": "cf1c4d5"}
+WARP_INST_MEASURED = {"spectral": "2f7be33", "plain": "3d152ab", "plain_wg": "cf1c4d5"}
 KERNEL = {"plain": "ncs_warp_kernel", "plain_wg": "ncs_plain_kernel",
-          "spectral": "ncs_spectral_kernel", "tc_tf32": "ncs_tc_kernel<TF32>",
+          "spectral": "ncs_pair_kernel", "tc_tf32": "ncs_tc_kernel<TF32>",
           "tc_bf16x3": "ncs_tc_kernel<BF16x3>"}
 # Tensor-core forms: MMA FLOPs executed per tile and pass (one transform pair),
 # from the four GEMM stages over 8 tiles (M = 128): stage 1 N 16 x K 16,
@@ -753,7 +753,7 @@ def run_ours(args, world, rank, local):
         warm = {"network": "4 x conv3x3 2-32-32-32-1, ReLU, %d params (%s on the tensor "
                            "cores)" % (warmstart.N_PARAMS, "E4M3" if fp8 else "BF16"),
                 "kernels": "ncsb::nettc::infer_tc<%s> (tcgen05, %s -> FP32 in TMEM), "
-                           "ncs_spectral_kernel<.., Warm>"
+                           "ncs_pair_kernel<.., Warm>"
                            % (("F8", "kind::f8f6f4 E4M3 x E4M3") if fp8
                               else ("BF16", "kind::f16 BF16 x BF16")),
                 "precision": args.warm_precision,
@@ -1060,7 +1060,7 @@ def run_mixed(args, world, rank, local):
         i1.record(stream)
         torch.cuda.synchronize()
         warm = {"kernels": "ncsb::nettc::infer_tc<%s> over the batch's stack descriptors, "
-                           "then ncs_spectral_kernel<.., Warm, Batch>, one CUDA graph"
+                           "then ncs_pair_kernel<.., Warm, Batch>, one CUDA graph"
                            % ("F8" if fp8 else "BF16"),
                 "precision": args.warm_precision,
                 "ms_per_step": w_ms, "ms_infer": i0.elapsed_time(i1),

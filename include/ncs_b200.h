@@ -61,8 +61,9 @@ extern "C" {
 /* Solver forms. */
 #define NCSB_MODE_PLAIN 0     /* FP32 SIMT, one warp per tile, in-register/smem FFT */
 #define NCSB_MODE_PLAIN_WG 1  /* FP32 SIMT, one warp group per tile (comparison form) */
-#define NCSB_MODE_SPECTRAL 2  /* FP32 SIMT, one warp per tile, L-BFGS with the spectral
-                                 initial inverse Hessian (lambda I + 2 alpha Q)^-1; m <= 4 */
+#define NCSB_MODE_SPECTRAL 2  /* FP32 SIMT, two tiles per warp at m = 1 and one above,
+                                 L-BFGS with the spectral initial inverse Hessian
+                                 (lambda I + 2 alpha Q)^-1; m <= 4 */
 /* Tensor-core forms: the spectral form's algorithm with every 16x16 transform
    of the noise term Q u = (1/256) F^H diag(M^2) F u (and of the initial
    inverse Hessian) done as four tcgen05 GEMMs over 8 tiles at a time, FP32
@@ -81,15 +82,17 @@ typedef struct {
     int32_t m;         /* history pairs, 1..8, at most 4 in the spectral form (ncs.cu M = 8;
                           libLBFGS m = 6; default 1: NCS tiles need the same number of
                           iterations for every m measured, 1..8 in the plain form and
-                          1..4 in the spectral one, and fewer pairs cost less -- the
-                          spectral solve measured about 6 % slower at m = 2 than at
-                          m = 1) */
+                          1..4 in the spectral one, and fewer pairs cost less; the
+                          spectral form runs two tiles per warp at m = 1 and one above
+                          (200 frames of 512 x 512: 1.31 ms at m = 1, 2.0 ms with one
+                          tile per warp) */
     double epsilon;    /* stop when ||g|| <= epsilon * max(1, ||u||)
                           (ncs.cu EPSILON = 1e-4; libLBFGS epsilon = 1e-5) */
     double c1;         /* Armijo constant (ncs.cu C_1 = 1e-4) */
     double min_step;   /* line search gives up below this step (ncs.cu MIN_STEP 1e-6) */
     int32_t mode;      /* NCSB_MODE_* */
-    int32_t ctas_per_sm; /* persistent grid: resident CTAs per SM, 0 = occupancy max */
+    int32_t ctas_per_sm; /* persistent grid: resident CTAs per SM, 0 = occupancy max (the
+                            spectral form at m = 1 takes no more than that, 3) */
 } ncsb_params;
 
 typedef struct ncsb_handle ncsb_handle;

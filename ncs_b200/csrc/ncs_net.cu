@@ -3,8 +3,9 @@
 // for the L-BFGS solve (include/ncs_b200.h, "learned warm start").  Forward,
 // weight gradient, input gradient (forward pass with flipped weights), ReLU
 // backward, MSE loss gradient, Adam, and a fused whole-network inference
-// kernel that cuts tiles straight from the stack.  FP32 SIMT throughout; one
-// 16x16 tile is one image, zero-padded at its border.
+// kernel that cuts tiles straight from the stack.  FP32 SIMT throughout, the
+// 32 -> 32 layers as Winograd convolutions (ncs_wino.cuh); one 16x16 tile is one
+// image, zero-padded at its border.
 //
 // Layouts: activations [n][c][16][16] in global memory; in shared memory one
 // channel is an 18x18 zero-bordered plane with a channel stride of kCS = 325

@@ -17,7 +17,7 @@
 // a lane to share each row with three others.
 //
 // What bounds it (stack512, 200 x 512^2): instruction issue and FP32 time in
-// turn, 58 % of the issue slots and 46 % of the FMA pipe at 12 warps per SM, with
+// turn, 59 % of the issue slots and 46 % of the FMA pipe at 12 warps per SM, with
 // waits on fixed latencies and on instruction fetch between.  A pass takes 1,095
 // warp instructions for two tiles, where one tile per warp took 1,004 for one:
 // the lane's own transforms replace 47 % of those, and every reduction and
@@ -974,15 +974,15 @@ ncs_pair_kernel(const SolveArgs a, const int one_wave) {
 
 namespace {
 
-// CTAs per SM: 3 (12 warps, 24 tiles, 168 registers).  On stack512 3 CTAs ran
-// 1.37 ms; 2 (no spills, 8 warps) 1.56 ms; 4 (128 registers, 200 B spilled)
-// 1.62 ms.
+// CTAs per SM: 3 (12 warps, 24 tiles, 168 registers).  On stack512, in an earlier
+// state of the kernel, 3 CTAs ran 1.37 ms (1.31 now); 2 (no spills, 8 warps) 1.56
+// ms; 4 (128 registers, 200 B spilled) 1.62 ms.
 constexpr int kPairBlocks = 3;
 
 using PairFn = void (*)(SolveArgs, int);
 
 // Launches of this many waves draw ahead to the end: the tail is short there
-// and the plainer loop compiles to the faster pass (stack512, 7.7 waves:
+// and the plainer loop compiles to the faster pass (stack512, 77 waves:
 // 1,306 us against 1,326).  Launches with proposals gained at every size
 // (512 frames of 512 x 512: 1,287 -> 1,279 us).
 constexpr long long kAheadWaves = 4;

@@ -204,7 +204,7 @@ __device__ __forceinline__ void tile_to_planes(const float4 (&v)[4], float* plan
 }
 
 // The kernels of a training step.  2048 tiles take 0.14 ms a layer here and 0.13
-// ms in wgrad (direct kernels: 0.56 and 0.46 ms); a step 2.91 -> 0.94 ms, its
+// ms in wgrad (direct kernels: 0.38 and 0.32 ms); a step 2.91 -> 0.94 ms, its
 // gradient's error against FP64 6.5e-7 -> 3.7e-7.
 //
 // y = conv(x, wt) + b per tile (b may be null), then ReLU (RELU), or the gradient
