@@ -982,9 +982,11 @@ constexpr int kPairBlocks = 3;
 using PairFn = void (*)(SolveArgs, int);
 
 // Launches of this many waves draw ahead to the end: the tail is short there
-// and the plainer loop compiles to the faster pass (stack512, 77 waves:
-// 1,306 us against 1,326).  Launches with proposals gained at every size
-// (512 frames of 512 x 512: 1,287 -> 1,279 us).
+// and the plainer loop compiles to the faster pass (stack512, 77 waves: 1,306
+// us against 1,326; at 11 waves, 60 x 411 x 301 raw counts, 226 either way; at
+// 3.7 waves 77.0 against 75.7).  Launches with proposals draw late at every size:
+// theirs gained at 19 waves too (50 x 512 x 512, inference included: 1,285 ->
+// 1,279 us).
 constexpr long long kAheadWaves = 4;
 
 PairFn pair_variant(bool warm, bool batch, bool late) {
