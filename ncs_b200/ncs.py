@@ -111,13 +111,16 @@ class Solver:
         with _on_device(self.device):
             self._scratch = torch.empty(_lib.HANDLE_SCRATCH_BYTES, dtype=torch.uint8,
                                         device=self.device)
-            torch.cuda.current_stream(self.device).synchronize()
+            alloc = torch.cuda.current_stream(self.device)
+            alloc.synchronize()
             rc = self.lib.ncsb_create_with_scratch(
                 ctypes.byref(self._handle), ctypes.byref(self.params), _ptr(self._scratch),
                 _lib.HANDLE_SCRATCH_BYTES)
         if rc != _lib.NCSB_OK:
             raise RuntimeError("ncsb_create failed with code %d" % rc)
         self.mask_shifted = None
+        # streams in whose order the scratch block may be reused
+        self._scratch_streams = {alloc.cuda_stream}
 
     def _set(self, **kw):
         for k, v in kw.items():
@@ -150,6 +153,16 @@ class Solver:
     def set_otf_mask(self, otf_mask_centred):
         """Centred mask (DC in the middle), fftshifted here (ncs.py:197)."""
         self.set_otf_mask_shifted(numpy.fft.fftshift(numpy.asarray(otf_mask_centred)))
+
+    def _launch_stream(self, stream, *tensors):
+        """launch_stream, and the handle's scratch recorded on the stream: a
+        launch reads it, so the block must not pass to other work before the
+        launch is done, whatever stream the solver was built on."""
+        s = launch_stream(stream, self.device, *tensors)
+        if s.cuda_stream not in self._scratch_streams:
+            self._scratch.record_stream(s)
+            self._scratch_streams.add(s.cuda_stream)
+        return s
 
     def _tensor(self, x, name, shape=None):
         if not isinstance(x, torch.Tensor) or not x.is_cuda:
@@ -196,7 +209,7 @@ class Solver:
             if tile_stats != "status":
                 cost = torch.empty(n, dtype=torch.float64, device=self.device)
                 evals = torch.empty(n, dtype=torch.int32, device=self.device)
-        s = launch_stream(stream, self.device, self._scratch, images, gamma, out, iters, status, cost, evals)
+        s = self._launch_stream(stream, images, gamma, out, iters, status, cost, evals)
         with _on_device(self.device):
             self._check(self.lib.ncsb_reduce_noise(
                 self._handle, _ptr(images), T, H, W, _ptr(gamma), per_frame, _ptr(out),
@@ -240,8 +253,8 @@ class Solver:
             cost = torch.empty(n, dtype=torch.float64, device=self.device)
             evals = torch.empty(n, dtype=torch.int32, device=self.device)
         start = torch.empty(n, dtype=torch.int32, device=self.device)
-        s = launch_stream(stream, self.device, self._scratch, images, gamma, u0_tiles, out, iters, status, cost,
-                          evals, start)
+        s = self._launch_stream(stream, images, gamma, u0_tiles, out, iters, status, cost, evals,
+                                start)
         with _on_device(self.device):
             self._check(self.lib.ncsb_reduce_noise_start(
                 self._handle, _ptr(images), T, H, W, _ptr(gamma), per_frame, _ptr(u0_tiles),
@@ -303,7 +316,7 @@ class Solver:
             n = self.num_tiles(T, H, W)
             st = [torch.empty(n, dtype=torch.int32, device=self.device) for _ in range(3)]
             cost = torch.empty(n, dtype=torch.float64, device=self.device)
-        s = launch_stream(stream, self.device, self._scratch, adu, out, cost, *st, *keep)
+        s = self._launch_stream(stream, adu, out, cost, *st, *keep)
         with _on_device(self.device):
             self._check(self.lib.ncsb_reduce_noise_adu_typed(
                 self._handle, _ptr(adu), _ADU_TYPES[adu.dtype], T, H, W, ctypes.byref(cal),
@@ -340,7 +353,7 @@ class Solver:
         elif (out.device.type != "cpu" or out.dtype != torch.float32
               or tuple(out.shape) != (T, H, W) or not out.is_contiguous()):
             raise ValueError("out must be a contiguous float32 host tensor [T, H, W]")
-        s = launch_stream(stream, self.device, self._scratch, *keep)
+        s = self._launch_stream(stream, *keep)
         with _on_device(self.device):
             self._check(self.lib.ncsb_reduce_noise_adu_host(
                 self._handle, _ptr(h_in), _ADU_TYPES[h_in.dtype], T, H, W, ctypes.byref(cal),
@@ -412,8 +425,8 @@ class Solver:
         if u0_tiles is not None:
             u0_tiles = self._tensor(u0_tiles, "u0_tiles", (self.batch_tiles, 16, 16))
         st = stats or {}
-        s = launch_stream(stream, self.device, self._scratch, u0_tiles, *st.values(),
-                          *[t for stack in self._batch for t in stack])
+        s = self._launch_stream(stream, u0_tiles, *st.values(),
+                                *[t for stack in self._batch for t in stack])
         with _on_device(self.device):
             self._check(self.lib.ncsb_batch_reduce_noise(
                 self._handle, _ptr(u0_tiles), _ptr(st.get("iters")), _ptr(st.get("status")),
@@ -468,7 +481,7 @@ class Solver:
         elif (out.device.type != "cpu" or out.dtype != torch.float32
               or tuple(out.shape) != (T, H, W) or not out.is_contiguous()):
             raise ValueError("out must be a contiguous float32 host tensor [T, H, W]")
-        s = launch_stream(stream, self.device, self._scratch)
+        s = self._launch_stream(stream)
         with _on_device(self.device):
             self._check(self.lib.ncsb_reduce_noise_host(
                 self._handle, _ptr(h_in), T, H, W, _ptr(h_g), per_frame, _ptr(out),
@@ -490,7 +503,7 @@ class Solver:
         status = torch.empty(n, dtype=torch.int32, device=self.device)
         cost = torch.empty(n, dtype=torch.float64, device=self.device)
         evals = torch.empty(n, dtype=torch.int32, device=self.device)
-        s = launch_stream(stream, self.device, self._scratch, data, gamma, u0, u, iters, status, cost, evals)
+        s = self._launch_stream(stream, data, gamma, u0, u, iters, status, cost, evals)
         with _on_device(self.device):
             self._check(self.lib.ncsb_solve_tiles(
                 self._handle, _ptr(data), _ptr(gamma), _ptr(u0), n, _ptr(u), _ptr(iters),

@@ -1,0 +1,81 @@
+"""CPU test of the lifetime of a Solver's device scratch (mask table, work
+counter): a launch on a stream other than the one the scratch was allocated on
+records the block there, also when that stream is simply the current one, so
+that dropping the Solver does not hand the block to other work while the launch
+may still read it.  Fake streams, tensors and library: no GPU is needed."""
+import contextlib
+
+import pytest
+import torch
+
+
+class Stream:
+    def __init__(self, handle):
+        self.cuda_stream = handle
+
+    def wait_stream(self, other):
+        pass
+
+    def synchronize(self):
+        pass
+
+
+class FakeCuda(torch.Tensor):
+    recorded = []
+
+    @property
+    def is_cuda(self):
+        return True
+
+    @property
+    def device(self):
+        return torch.device("cuda", 0)
+
+    def record_stream(self, s):
+        FakeCuda.recorded.append((self.data_ptr(), s))
+
+
+def fake(*shape):
+    return torch.Tensor._make_subclass(FakeCuda, torch.zeros(*shape))
+
+
+class Lib:
+    def __getattr__(self, name):
+        return lambda *a: 0
+
+
+@pytest.fixture
+def solver(monkeypatch):
+    from ncs_b200 import _lib, ncs
+    current = [Stream(7)]
+    monkeypatch.setattr(_lib, "load", Lib)
+    monkeypatch.setattr(_lib, "default_params", _lib.NcsbParams)
+    monkeypatch.setattr(ncs, "_on_device", lambda device: contextlib.nullcontext())
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: 0)
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda device=None: current[0])
+    monkeypatch.setattr(torch.cuda, "stream", lambda s: contextlib.nullcontext())
+    monkeypatch.setattr(torch.cuda, "Stream", lambda *a, **k: Stream(99))
+    real = torch.empty
+    monkeypatch.setattr(torch, "empty",
+                        lambda *a, device=None, **k: torch.Tensor._make_subclass(FakeCuda, real(*a, **k)))
+    FakeCuda.recorded = []
+    s = ncs.Solver()
+    s._current = current
+    return s
+
+
+@pytest.mark.parametrize("explicit", [False, True])
+def test_launch_on_another_stream_records_the_scratch(solver, explicit):
+    x, g, tiles = fake(1, 16, 16), fake(16, 16), fake(4, 16, 16)
+    u0 = fake(solver.num_tiles(1, 16, 16), 16, 16)
+    at = solver._scratch.data_ptr()
+    for call in (lambda **k: solver.reduce_noise(x, g, **k),
+                 lambda **k: solver.solve_tiles(tiles, tiles, **k),
+                 lambda **k: solver.reduce_noise_from(x, g, u0, **k)):
+        b = Stream(8 + len(FakeCuda.recorded))  # each on a stream of its own
+        if explicit:
+            call(stream=b)
+        else:
+            solver._current[0] = b
+            call()
+        assert (at, b) in FakeCuda.recorded
