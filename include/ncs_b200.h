@@ -107,7 +107,9 @@ int ncsb_create(ncsb_handle **out, const ncsb_params *p);
 /* The same with the handle's device scratch (mask table, work counter) given by
  * the caller, e.g. from its own caching allocator: at least
  * NCSB_HANDLE_SCRATCH_BYTES, 16-byte aligned, idle when this is called, and
- * left alone while the handle exists and its launches run. */
+ * left alone while the handle exists and its launches run.  ncsb_destroy waits
+ * for the device if a launch was captured into a graph, whose replays may run on
+ * any stream. */
 #define NCSB_HANDLE_SCRATCH_BYTES 2048
 int ncsb_create_with_scratch(ncsb_handle **out, const ncsb_params *p, void *scratch, size_t bytes);
 int ncsb_set_params(ncsb_handle *h, const ncsb_params *p);

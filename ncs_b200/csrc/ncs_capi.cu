@@ -114,6 +114,7 @@ struct ncsb_handle {
     bool has_mask = false;
     // Device scratch (NCSB_HANDLE_SCRATCH_BYTES), allocated here or the caller's:
     bool own_scratch = false;
+    bool captured = false;  // a launch of this handle went into a stream capture
     float* d_msq = nullptr;                 // [256] M^2/256, natural [kr][kc] order
     unsigned long long* d_queue = nullptr;  // work counter
     int32_t* d_flag = nullptr;              // tensor-core forms: 1 after a wait ran out
@@ -205,6 +206,9 @@ void lane_layout(const float nat[256], float* out) {
 // queue: the work counter of this launch (default: the handle's own)
 int launch(ncsb_handle* h, ncsb::SolveArgs& a, cudaStream_t s, unsigned long long* queue = nullptr) {
     if (!queue) queue = h->d_queue;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (!h->captured && cudaStreamIsCapturing(s, &cap) == cudaSuccess)
+        h->captured = cap != cudaStreamCaptureStatusNone;
     // the default form at m = 1 runs two tiles per warp (ncs_pair.cu); a launch
     // that gives each pair its own warp leaves the work counter alone
     const bool pair = h->p.mode == NCSB_MODE_SPECTRAL && h->p.m <= 1;
@@ -325,6 +329,15 @@ int ncsb_destroy(ncsb_handle* h) {
     if (!h) return NCSB_EINVAL;
     destroy_pipe(h->pipe);
     cudaFree(h->d_adu);
+    // a captured launch may be replayed on any stream, so the caller cannot know
+    // when its scratch is idle: wait for the device, as cudaFree does
+    if (h->captured && !h->own_scratch) {
+        int dev = h->device;
+        cudaGetDevice(&dev);
+        if (dev != h->device) cudaSetDevice(h->device);
+        cudaDeviceSynchronize();
+        if (dev != h->device) cudaSetDevice(dev);
+    }
     if (h->own_scratch) cudaFree(h->d_msq);
     cudaFree(h->d_stacks);
     cudaFree(h->d_mk_lane);

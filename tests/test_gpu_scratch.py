@@ -46,3 +46,27 @@ def test_solver_dropped_while_a_launch_on_another_stream_waits(cuda_ok, call):
     torch.cuda.synchronize()
     assert torch.equal(out, want)
     del others
+
+
+def test_solver_dropped_while_a_replayed_graph_waits(cuda_ok):
+    mask = create_otf_mask_shifted()
+    im, gam = stack()
+    want = solver(mask).reduce_noise(im, gam)
+    s = solver(mask)
+    out = torch.empty_like(im)
+    s.reduce_noise(im, gam, out=out)
+    torch.cuda.synchronize()
+    out.zero_()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        s.reduce_noise(im, gam, out=out)
+    torch.cuda.synchronize()
+    side = torch.cuda.Stream()  # not the stream of the capture
+    with torch.cuda.stream(side):
+        torch.cuda._sleep(SLEEP)
+        graph.replay()
+    del s
+    others = [solver(0.5 * mask) for _ in range(4)]
+    torch.cuda.synchronize()
+    assert torch.equal(out, want)
+    del others
