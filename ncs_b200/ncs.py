@@ -74,6 +74,17 @@ def launch_stream(stream, device, *tensors):
     return stream
 
 
+_scratch_stream_of = {}  # device index -> stream
+
+
+def _scratch_stream(device):
+    """The stream on which handle scratch of a device is allocated."""
+    s = _scratch_stream_of.get(device.index)
+    if s is None:
+        s = _scratch_stream_of.setdefault(device.index, torch.cuda.Stream(device))
+    return s
+
+
 _ADU_TYPES = {torch.float32: _lib.ADU_F32, torch.uint16: _lib.ADU_U16, torch.uint8: _lib.ADU_U8}
 
 _MODES = {"plain": _lib.MODE_PLAIN, "plain_wg": _lib.MODE_PLAIN_WG,
@@ -106,12 +117,15 @@ class Solver:
         self._set(alpha=alpha, max_iters=max_iters, m=m, epsilon=epsilon, c1=c1,
                   min_step=min_step, mode=mode, ctas_per_sm=ctas_per_sm)
         # The handle's scratch comes from the caching allocator (three cudaMalloc
-        # and cudaFree calls took 1 ms of a short-lived solver); earlier work on
-        # the current stream may still use the block, so it is waited for.
+        # and cudaFree calls took 1 ms of a short-lived solver), allocated on a
+        # stream that only scratch is allocated on.  Every launch stream is recorded
+        # on it, so a block that is handed out is idle whatever is queued on the
+        # current stream; the wait covers other users of the pooled stream.
         with _on_device(self.device):
-            self._scratch = torch.empty(_lib.HANDLE_SCRATCH_BYTES, dtype=torch.uint8,
-                                        device=self.device)
-            alloc = torch.cuda.current_stream(self.device)
+            alloc = _scratch_stream(self.device)
+            with torch.cuda.stream(alloc):
+                self._scratch = torch.empty(_lib.HANDLE_SCRATCH_BYTES, dtype=torch.uint8,
+                                            device=self.device)
             alloc.synchronize()
             rc = self.lib.ncsb_create_with_scratch(
                 ctypes.byref(self._handle), ctypes.byref(self.params), _ptr(self._scratch),

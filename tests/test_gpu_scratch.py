@@ -70,3 +70,18 @@ def test_solver_dropped_while_a_replayed_graph_waits(cuda_ok):
     torch.cuda.synchronize()
     assert torch.equal(out, want)
     del others
+
+
+def test_building_a_solver_does_not_wait_for_queued_work(cuda_ok):
+    mask = create_otf_mask_shifted()
+    keep = solver(mask)  # the allocator's segment for scratch exists
+    side, end = torch.cuda.Stream(), torch.cuda.Event()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(side):
+        torch.cuda._sleep(SLEEP)
+        end.record()
+        s = solver(mask)
+    assert not end.query()
+    torch.cuda.synchronize()
+    im, gam = stack()
+    assert torch.equal(s.reduce_noise(im, gam), keep.reduce_noise(im, gam))
