@@ -416,7 +416,8 @@ int ncsb_net_conv_wgrad(const float *x, const float *dy, float *dwt, float *db, 
 
 /* Backward passes of a training step of n tiles.  Every [n][32][16][16] array is
  * 16-byte aligned; gradients and the loss are added to.
- * ncsb_net_conv_xgrad: input gradient dx of a 32 -> 32 layer with weights
+ * ncsb_net_conv_xgrad: input gradient dx (no other argument's memory) of a
+ * 32 -> 32 layer with weights
  * wt [32][9][32] from its output gradient dy, zero where act <= 0 (act: the
  * layer's input, a ReLU's output; NULL: no mask).
  * ncsb_net_last_layer: from a [n][32][16][16] (the last layer's input, a ReLU's

@@ -564,7 +564,7 @@ int ncsb_net_conv_fwd(const float* x, const float* wt, const float* b, float* y,
     cudaStream_t s = (cudaStream_t)stream;
     if (cin == 2 && cout == 32)
         return relu ? launch_fwd<2, 32, true>(x, wt, b, y, n, s) : launch_fwd<2, 32, false>(x, wt, b, y, n, s);
-    if (cin == 32 && cout == 32 && aligned16(x, y, y))
+    if (cin == 32 && cout == 32 && aligned16(x, y, y) && x != y)
         return relu ? launch_wino<true, false, false>(x, wt, b, nullptr, y, n, s)
                     : launch_wino<false, false, false>(x, wt, b, nullptr, y, n, s);
     if (cin == 32 && cout == 32)

@@ -203,8 +203,63 @@ __device__ __forceinline__ void tile_to_planes(const float4 (&v)[4], float* plan
     }
 }
 
+// The transforms add up to four inputs, so an infinity turns every output of its
+// patches into NaN, where the direct form has infinities at the neighbours alone, and
+// large values may overflow.  conv and wgrad watch their results for either and, rarely,
+// take those tiles again in the direct form: tiles or weights with a value past kWild
+// (NaN included), below which nothing overflows.
+constexpr float kWild = 1.0e15f;
+// |x| as bits: ordered as |x|, NaN above all
+__device__ __forceinline__ int abs_bits(float x) { return __float_as_int(x) & 0x7fffffff; }
+constexpr int kInfBits = 0x7f800000;
+__device__ __noinline__ bool wild(const float* __restrict__ x, int n) {  // for the CTA
+    bool w = false;
+#pragma unroll 1
+    for (int i = threadIdx.x; i < n; i += kThreads) w = w || !(fabsf(x[i]) <= kWild);
+    return __syncthreads_or(w) != 0;
+}
+
+// The layer of one tile (pointers to its kC x 256 values) in the direct form.
+__device__ __noinline__ void direct_conv(const float* __restrict__ x, const float* __restrict__ wt,
+                                         const float* __restrict__ b, const float* __restrict__ act,
+                                         float* __restrict__ y, bool relu, bool flip) {
+#pragma unroll 1
+    for (int i = threadIdx.x; i < kC * 256; i += kThreads) {
+        const int co = i >> 8, r = (i >> 4) & 15, c = i & 15;
+        float acc = b ? b[co] : 0.0f;
+#pragma unroll 1
+        for (int ci = 0; ci < kC; ++ci)
+#pragma unroll 1
+            for (int k = 0; k < 9; ++k) {
+                const int yy = r + k / 3 - 1, xx = c + k % 3 - 1;
+                const float v = (unsigned)yy < 16u && (unsigned)xx < 16u
+                                    ? x[ci * 256 + yy * 16 + xx] : 0.0f;
+                acc = fmaf(flip ? wt[(co * 9 + 8 - k) * kC + ci] : wt[(ci * 9 + k) * kC + co], v, acc);
+            }
+        if (relu) acc = fmaxf(acc, 0.0f);
+        y[i] = act && !(act[i] > 0.0f) ? 0.0f : acc;
+    }
+}
+
+// The weight gradient of one tile, added to dwt.
+__device__ __noinline__ void direct_wgrad(const float* __restrict__ x, const float* __restrict__ dy,
+                                          float* __restrict__ dwt) {
+#pragma unroll 1
+    for (int i = threadIdx.x; i < 9 * kC * kC; i += kThreads) {
+        const int co = i & 31, k = (i >> 5) % 9, ci = i / (9 * kC);
+        double s = 0.0;
+#pragma unroll 1
+        for (int p = 0; p < 256; ++p) {
+            const int yy = (p >> 4) + k / 3 - 1, xx = (p & 15) + k % 3 - 1;
+            const float v = (unsigned)yy < 16u && (unsigned)xx < 16u ? x[ci * 256 + yy * 16 + xx] : 0.0f;
+            s = fma((double)v, (double)dy[co * 256 + p], s);
+        }
+        atomicAdd(dwt + i, (float)s);
+    }
+}
+
 // The kernels of a training step.  2048 tiles take 0.14 ms a layer here and 0.13
-// ms in wgrad (direct kernels: 0.38 and 0.32 ms); a step 2.91 -> 0.94 ms, its
+// ms in wgrad (direct kernels: 0.38 and 0.32 ms); a step 2.91 -> 0.95 ms, its
 // gradient's error against FP64 6.5e-7 -> 3.7e-7.
 //
 // y = conv(x, wt) + b per tile (b may be null), then ReLU (RELU), or the gradient
@@ -232,6 +287,8 @@ __global__ void __launch_bounds__(kThreads) conv(const float* __restrict__ x,
         for (int i = t; i < 2 * kPlane; i += kThreads) fp[i] = 0.0f;
     weights(U, wt, FLIP);
     const float bias = b ? b[lane] : 0.0f;
+    __shared__ int odd;  // an output of this CTA is not finite
+    if (t == 0) odd = 0;
     float tot[FIRST ? 19 : 1] = {};  // FIRST: this lane's channel: 18 weights and the bias
     float4 next[4];
     int tile = blockIdx.x;
@@ -246,6 +303,12 @@ __global__ void __launch_bounds__(kThreads) conv(const float* __restrict__ x,
         __syncthreads();
         float out[16];
         layer<kCp>(planes, U, vm, bias, out);
+        if (!FIRST) {
+            int top = 0;
+#pragma unroll
+            for (int k = 0; k < 16; ++k) top = max(top, abs_bits(out[k]));
+            if (top >= kInfBits) odd = 1;
+        }
         if (RELU) {
 #pragma unroll
             for (int k = 0; k < 16; ++k) out[k] = fmaxf(out[k], 0.0f);
@@ -308,6 +371,17 @@ __global__ void __launch_bounds__(kThreads) conv(const float* __restrict__ x,
             }
 #pragma unroll
             for (int k = 0; k < 18; ++k) tot[k] += acc[k];
+        }
+    }
+    if (!FIRST) {
+        __syncthreads();
+        if (odd) {
+            const bool all = wild(wt, 9 * kC * kC);
+            for (tile = blockIdx.x; tile < n; tile += gridDim.x) {
+                const size_t at = (size_t)tile * kC * 256;
+                if (wild(x + at, kC * 256) || all)
+                    direct_conv(x + at, wt, b, act ? act + at : nullptr, y + at, RELU, FLIP);
+            }
         }
     }
     if (FIRST) {
@@ -414,6 +488,15 @@ __global__ void __launch_bounds__(kThreads) wgrad(const float* __restrict__ x,
             __syncthreads();
         }
     }
+    int top = 0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+        top = max(top, max(max(abs_bits(acc[i][0].x), abs_bits(acc[i][0].y)),
+                           max(abs_bits(acc[i][1].x), abs_bits(acc[i][1].y))));
+    const bool odd = __syncthreads_or(top >= kInfBits) != 0;
+    if (odd)
+        for (tile = blockIdx.x; tile < n; tile += gridDim.x)
+            direct_wgrad(x + (size_t)tile * kC * 256, dy + (size_t)tile * kC * 256, dwt);
     // M[point][ci][co] through shared memory (V and dY's 16 x 1024 floats)
     float* M = V;
 #pragma unroll
@@ -422,7 +505,7 @@ __global__ void __launch_bounds__(kThreads) wgrad(const float* __restrict__ x,
             make_float4(acc[i][0].x, acc[i][0].y, acc[i][1].x, acc[i][1].y);
     reinterpret_cast<double*>(gs)[t] = bsum;  // [warp][channel]
     __syncthreads();
-    for (int idx = t; idx < kC * kC; idx += kThreads) {
+    for (int idx = odd ? kC * kC : t; idx < kC * kC; idx += kThreads) {
         const int ci = idx >> 5, co = idx & 31;
         float m[4][4], r[3][4];
 #pragma unroll
