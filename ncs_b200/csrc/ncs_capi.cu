@@ -801,7 +801,7 @@ int ncsb_batch_set(ncsb_handle* h, const ncsb_stack* stacks, int n_stacks) {
     h->batch_tiles = total;
     // resolve the kernel variants' attributes now, outside any stream capture
     for (const bool warm : {false, true}) {
-        ncsb::spectral_max_ctas_per_sm(h->p.m, 0, warm, true);
+        if (h->p.m > 1) ncsb::spectral_max_ctas_per_sm(h->p.m, 0, warm, true);
         e = ncsb::pair_prepare(warm, true);
         if (e != cudaSuccess) return cuda_fail(h, e, "kernel attributes");
     }
