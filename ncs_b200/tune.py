@@ -2,8 +2,8 @@
 
 The kernels pull tiles from a device-side queue, so the work per CTA adapts
 by itself; what a launch fixes is how many CTAs (four warps, at m = 1
-two tiles and above it one per warp at a time) stay resident per SM and the L-BFGS history size m.  Both
-change speed but not the result's accuracy (the stopping rule is the same),
+two tiles and above it one per warp at a time) stay resident per SM and the
+L-BFGS history size m.  Both change speed but not the result's accuracy (the stopping rule is the same),
 so the tuner times every candidate on the caller's own workload with CUDA
 events and keeps the fastest.  Results are cached per workload key in
 memory and, optionally, in a JSON file.
@@ -16,7 +16,9 @@ import os
 
 import torch
 
-DEFAULT_CANDIDATES = tuple({"ctas_per_sm": c, "m": m} for c in (2, 3, 4) for m in (1, 2, 4))
+# m = 1 takes at most 3 CTAs per SM (4 is the same launch)
+DEFAULT_CANDIDATES = tuple({"ctas_per_sm": c, "m": m} for c in (2, 3, 4) for m in (1, 2, 4)
+                           if c <= 3 or m > 1)
 
 _cache = {}
 
