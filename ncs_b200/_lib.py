@@ -114,8 +114,9 @@ HANDLE_SCRATCH_BYTES = 2048
 
 # Every symbol include/ncs_b200.h declares (checked by the tests).
 EXPORTS = [
-    "ncsb_default_params", "ncsb_create", "ncsb_create_with_scratch", "ncsb_set_params", "ncsb_destroy", "ncsb_last_error",
-    "ncsb_set_otf_mask", "ncsb_num_tiles", "ncsb_reduce_noise", "ncsb_solve_tiles",
+    "ncsb_default_params", "ncsb_create", "ncsb_create_with_scratch", "ncsb_set_params",
+    "ncsb_destroy", "ncsb_last_error", "ncsb_set_otf_mask", "ncsb_num_tiles",
+    "ncsb_reduce_noise", "ncsb_solve_tiles",
     "ncsb_reduce_noise_noalloc", "ncsb_reduce_noise_start",
     "ncsb_net_param_count", "ncsb_net_conv_fwd", "ncsb_net_conv_wgrad", "ncsb_net_flip",
     "ncsb_net_conv_xgrad", "ncsb_net_last_layer", "ncsb_net_first_layers_grad",

@@ -292,12 +292,12 @@ struct InferSrc {
 
 // Shared memory of the fused inference, in floats: both hidden layers'
 // transformed weights, the activation planes, the Winograd exchange buffer, then
-// the first and last layer's weights, the biases, the input planes and the sums
+// the first and last layer's weights and biases, the input planes and the sums
 // of the tile scale.  The last layer's weights are [ci][12] (9 taps).
 struct InferSmem {
     static constexpr int u2 = 0, u3 = u2 + wino::kU, planes = u3 + wino::kU,
                          vm = planes + wino::kPlanes, w1 = vm + wino::kV(16), b1 = w1 + 2 * 9 * kC,
-                         b2 = b1 + kC, b3 = b2 + kC, w4 = b3 + kC, b4 = w4 + 12 * kC,
+                         w4 = b1 + kC, b4 = w4 + 12 * kC,
                          xin = b4 + 4, red = xin + 2 * wino::kPlane, end = red + 16;
 };
 constexpr size_t kInferSmem = InferSmem::end * sizeof(float);

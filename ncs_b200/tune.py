@@ -3,9 +3,9 @@
 The kernels pull tiles from a device-side queue, so the work per CTA adapts
 by itself; what a launch fixes is how many CTAs (four warps, at m = 1
 two tiles and above it one per warp at a time) stay resident per SM and the
-L-BFGS history size m.  Both change speed but not the result's accuracy (the stopping rule is the same),
-so the tuner times every candidate on the caller's own workload with CUDA
-events and keeps the fastest.  Results are cached per workload key in
+L-BFGS history size m.  Both change speed but not the result's accuracy (the
+stopping rule is the same), so the tuner times every candidate on the caller's
+own workload with CUDA events and keeps the fastest.  Results are cached per workload key in
 memory and, optionally, in a JSON file.
 
 No counterpart in the reference, whose launch geometry is fixed

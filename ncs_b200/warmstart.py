@@ -101,12 +101,6 @@ class WarmStartNet:
         if rc != _lib.NCSB_OK:
             raise RuntimeError("%s failed with code %d" % (what, rc))
 
-    def _slices(self, vec):
-        out = []
-        for wo, nw, bo, nb in layer_offsets():
-            out.append((vec[wo:wo + nw], vec[bo:bo + nb]))
-        return out
-
     # ---- inference ----------------------------------------------------------
     def propose_stack(self, images, gamma, out=None, stream=None):
         """Proposals [n_tiles, 16, 16] for a [T, H, W] stack (gamma [H, W] or
