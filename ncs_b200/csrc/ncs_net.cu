@@ -309,7 +309,7 @@ constexpr int kInferThreads = 256;
 // of all layers took one float4 weight broadcast per 4 multiply-adds and was
 // bound by the shared-memory pipe (96 % busy): 20 x 512^2 frames 9.15 ms, this 3.72
 // ms (FMA pipe 51 %, shared memory 79 % of the time); error against FP64 3.1e-7
-// direct, 1.4e-7 this.
+// direct, 1.5e-7 this.
 __global__ void __launch_bounds__(kInferThreads) infer(const InferSrc src,
                                                         const float* __restrict__ params,
                                                         float* __restrict__ u0) {

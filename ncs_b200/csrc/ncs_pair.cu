@@ -18,7 +18,9 @@
 //
 // What bounds it (stack512, 200 x 512^2): instruction issue and FP32 time in
 // turn, 59 % of the issue slots and 46 % of the FMA pipe at 12 warps per SM, with
-// waits on fixed latencies and on instruction fetch between.  A pass takes 1,095
+// waits on fixed latencies and on instruction fetch between; the shared-memory path
+// is 56 % busy, mostly with the vectors kept there (160 wavefronts a pass, the
+// transposes 64).  A pass takes 1,095
 // warp instructions for two tiles, where one tile per warp took 1,004 for one:
 // the lane's own transforms replace 47 % of those, and every reduction and
 // per-tile decision serves two tiles.  2.01 -> 1.31 ms (sensor2048: 15.75 ->
@@ -215,8 +217,9 @@ __device__ __forceinline__ float tab_scale(int kr, int kc) {
 }
 
 // log1p(x) = 2 atanh(y), y = x / (2 + x).  2 atanh(y) / y as a polynomial in
-// y^2, minimax in relative error: 4e-9 for |y| <= 1/3 (x in -1/2 .. 1), and
-// 1e-8 for |y| <= 0.7 (x in -0.82 .. 4.7), which first iterations need.
+// y^2, fitted for the relative error: with these FP32 coefficients 8e-9 for
+// |y| <= 1/3 (x in -1/2 .. 1) and 2e-8 for |y| <= 0.7 (x in -0.82 .. 4.7), which
+// first iterations need; evaluated in FP32 1.3e-7 and 1.4e-7, its own roundings.
 constexpr float kNear = 1.0f / 3.0f, kFar = 0.7f;
 __device__ constexpr float kNearPoly[5] = {2.0f, 0.666663147f, 0.400249103f, 0.279606027f,
                                            0.281783351f};
@@ -491,7 +494,10 @@ ncs_pair_kernel(const SolveArgs a, const int one_wave) {
                 if (asym) {
                     // bins (kr, kc) and (kr, -kc) have weights a and b: the cos-cos
                     // and sin-sin coefficients mix, and so do cos-sin and sin-cos,
-                    // with P = (a + b) / 2 and N = (a - b) / 2
+                    // with P = (a + b) / 2 and N = (a - b) / 2.  A solve with such a mask
+                    // takes a tenth longer (200 x 512 x 512: 990 us radial, 1,087 so; one
+                    // tile per warp: 1,510 either way), a batch of 16 stacks 0.1 us more
+                    // with one of them, 4 of 56 with all
                     float wa[9];
 #pragma unroll
                     for (int k = 0; k < 9; ++k) wa[k] = w[k];
