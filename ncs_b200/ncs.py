@@ -135,6 +135,7 @@ class Solver:
         self.mask_shifted = None
         # streams in whose order the scratch block may be reused
         self._scratch_streams = {alloc.cuda_stream}
+        self._foreign = False
 
     def _set(self, **kw):
         for k, v in kw.items():
@@ -171,11 +172,17 @@ class Solver:
     def _launch_stream(self, stream, *tensors):
         """launch_stream, and the handle's scratch recorded on the stream: a
         launch reads it, so the block must not pass to other work before the
-        launch is done, whatever stream the solver was built on."""
+        launch is done, whatever stream the solver was built on.  Streams that
+        are not torch's own (their stream_id is the CUDA handle) may be gone by
+        then: after one of those, close() waits for the device instead."""
         s = launch_stream(stream, self.device, *tensors)
-        if s.cuda_stream not in self._scratch_streams:
-            self._scratch.record_stream(s)
-            self._scratch_streams.add(s.cuda_stream)
+        handle = s.cuda_stream
+        if handle not in self._scratch_streams:
+            if handle != 0 and s.stream_id == handle:
+                self._foreign = True
+            else:
+                self._scratch.record_stream(s)
+            self._scratch_streams.add(handle)
         return s
 
     def _tensor(self, x, name, shape=None):
@@ -527,6 +534,8 @@ class Solver:
 
     def close(self):
         if getattr(self, "_handle", None) and self._handle.value:
+            if self._foreign:
+                torch.cuda.synchronize(self.device)
             self.lib.ncsb_destroy(self._handle)
             self._handle = ctypes.c_void_p()
 

@@ -85,3 +85,21 @@ def test_building_a_solver_does_not_wait_for_queued_work(cuda_ok):
     torch.cuda.synchronize()
     im, gam = stack()
     assert torch.equal(s.reduce_noise(im, gam), keep.reduce_noise(im, gam))
+
+
+def test_solver_outlives_a_stream_that_is_not_torchs(cuda_ok):
+    import ctypes
+    mask = create_otf_mask_shifted()
+    im, gam = stack()
+    want = solver(mask).reduce_noise(im, gam)
+    s, out = solver(mask), torch.empty_like(im)
+    raw, rt = ctypes.c_ulonglong(0), torch.cuda.cudart()
+    assert int(rt.cudaStreamCreate(ctypes.addressof(raw))) == 0
+    torch.cuda.synchronize()
+    with torch.cuda.stream(torch.cuda.ExternalStream(raw.value)):
+        s.reduce_noise(im, gam, out=out)
+    torch.cuda.synchronize()
+    assert int(rt.cudaStreamDestroy(raw.value)) == 0
+    del s
+    assert torch.equal(out, want)
+    assert torch.equal(solver(mask).reduce_noise(im, gam), want)

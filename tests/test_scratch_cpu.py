@@ -10,8 +10,9 @@ import torch
 
 
 class Stream:
-    def __init__(self, handle):
+    def __init__(self, handle, foreign=False):
         self.cuda_stream = handle
+        self.stream_id = handle if foreign else 2 * handle + 1
 
     def wait_stream(self, other):
         pass
@@ -79,3 +80,16 @@ def test_launch_on_another_stream_records_the_scratch(solver, explicit):
             solver._current[0] = b
             call()
         assert (at, b) in FakeCuda.recorded
+
+
+def test_a_foreign_stream_is_waited_for_instead(solver, monkeypatch):
+    """An external stream may be destroyed before the Solver: nothing is recorded
+    on it, and close() waits for the device."""
+    waits = []
+    monkeypatch.setattr(torch.cuda, "synchronize", waits.append)
+    solver._handle.value = 1
+    solver._current[0] = Stream(1024, foreign=True)
+    solver.solve_tiles(fake(4, 16, 16), fake(4, 16, 16))
+    assert not FakeCuda.recorded
+    solver.close()
+    assert waits == [solver.device]
