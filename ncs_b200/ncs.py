@@ -74,15 +74,34 @@ def launch_stream(stream, device, *tensors):
     return stream
 
 
+def _foreign(stream):
+    """Whether a stream is not one of torch's own (an ExternalStream's id is its
+    CUDA handle): it may be destroyed while tensors are recorded on it."""
+    return stream.cuda_stream != 0 and stream.stream_id == stream.cuda_stream
+
+
 _scratch_stream_of = {}  # device index -> stream
 
 
-def _scratch_stream(device):
-    """The stream on which handle scratch of a device is allocated."""
-    s = _scratch_stream_of.get(device.index)
-    if s is None:
-        s = _scratch_stream_of.setdefault(device.index, torch.cuda.Stream(device))
-    return s
+def _scratch_block(device):
+    """A handle's device scratch from the caching allocator (three cudaMalloc and
+    cudaFree calls took 1 ms of a short-lived solver) and the stream that it was
+    allocated on.  Nothing may still use the block: the allocator only keeps the
+    order of that stream.  The current stream's blocks are idle when the stream is;
+    behind queued work the block comes from a stream on which nothing but scratch is
+    allocated, so that building a solver does not wait for the work."""
+    alloc = torch.cuda.current_stream(device)
+    if not torch.cuda.is_current_stream_capturing() and not _foreign(alloc):
+        block = torch.empty(_lib.HANDLE_SCRATCH_BYTES, dtype=torch.uint8, device=device)
+        if alloc.query():
+            return block, alloc
+    alloc = _scratch_stream_of.get(device.index)
+    if alloc is None:
+        alloc = _scratch_stream_of.setdefault(device.index, torch.cuda.Stream(device))
+    with torch.cuda.stream(alloc):
+        block = torch.empty(_lib.HANDLE_SCRATCH_BYTES, dtype=torch.uint8, device=device)
+    alloc.synchronize()  # other users of the pooled stream
+    return block, alloc
 
 
 _ADU_TYPES = {torch.float32: _lib.ADU_F32, torch.uint16: _lib.ADU_U16, torch.uint8: _lib.ADU_U8}
@@ -116,17 +135,8 @@ class Solver:
         self._handle = ctypes.c_void_p()
         self._set(alpha=alpha, max_iters=max_iters, m=m, epsilon=epsilon, c1=c1,
                   min_step=min_step, mode=mode, ctas_per_sm=ctas_per_sm)
-        # The handle's scratch comes from the caching allocator (three cudaMalloc
-        # and cudaFree calls took 1 ms of a short-lived solver), allocated on a
-        # stream that only scratch is allocated on.  Every launch stream is recorded
-        # on it, so a block that is handed out is idle whatever is queued on the
-        # current stream; the wait covers other users of the pooled stream.
         with _on_device(self.device):
-            alloc = _scratch_stream(self.device)
-            with torch.cuda.stream(alloc):
-                self._scratch = torch.empty(_lib.HANDLE_SCRATCH_BYTES, dtype=torch.uint8,
-                                            device=self.device)
-            alloc.synchronize()
+            self._scratch, alloc = _scratch_block(self.device)
             rc = self.lib.ncsb_create_with_scratch(
                 ctypes.byref(self._handle), ctypes.byref(self.params), _ptr(self._scratch),
                 _lib.HANDLE_SCRATCH_BYTES)
@@ -135,7 +145,7 @@ class Solver:
         self.mask_shifted = None
         # streams in whose order the scratch block may be reused
         self._scratch_streams = {alloc.cuda_stream}
-        self._foreign = False
+        self._wait_at_close = False
 
     def _set(self, **kw):
         for k, v in kw.items():
@@ -172,17 +182,16 @@ class Solver:
     def _launch_stream(self, stream, *tensors):
         """launch_stream, and the handle's scratch recorded on the stream: a
         launch reads it, so the block must not pass to other work before the
-        launch is done, whatever stream the solver was built on.  Streams that
-        are not torch's own (their stream_id is the CUDA handle) may be gone by
-        then: after one of those, close() waits for the device instead."""
+        launch is done, whatever stream the solver was built on.  A stream that is
+        not torch's may be gone by then: after one of those, close() waits for the
+        device instead."""
         s = launch_stream(stream, self.device, *tensors)
-        handle = s.cuda_stream
-        if handle not in self._scratch_streams:
-            if handle != 0 and s.stream_id == handle:
-                self._foreign = True
+        if s.cuda_stream not in self._scratch_streams:
+            if _foreign(s):
+                self._wait_at_close = True
             else:
                 self._scratch.record_stream(s)
-            self._scratch_streams.add(handle)
+            self._scratch_streams.add(s.cuda_stream)
         return s
 
     def _tensor(self, x, name, shape=None):
@@ -534,7 +543,7 @@ class Solver:
 
     def close(self):
         if getattr(self, "_handle", None) and self._handle.value:
-            if self._foreign:
+            if self._wait_at_close:
                 torch.cuda.synchronize(self.device)
             self.lib.ncsb_destroy(self._handle)
             self._handle = ctypes.c_void_p()

@@ -10,12 +10,17 @@ import torch
 
 
 class Stream:
+    busy = False
+
     def __init__(self, handle, foreign=False):
         self.cuda_stream = handle
         self.stream_id = handle if foreign else 2 * handle + 1
 
     def wait_stream(self, other):
         pass
+
+    def query(self):
+        return not self.busy
 
     def synchronize(self):
         pass
@@ -45,10 +50,13 @@ class Lib:
         return lambda *a: 0
 
 
-@pytest.fixture
-def solver(monkeypatch):
+@pytest.fixture(params=[False, True], ids=["idle", "busy"])
+def solver(monkeypatch, request):
     from ncs_b200 import _lib, ncs
     current = [Stream(7)]
+    current[0].busy = request.param  # then the block comes from another stream
+    monkeypatch.setattr(ncs, "_scratch_stream_of", {})
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
     monkeypatch.setattr(_lib, "load", Lib)
     monkeypatch.setattr(_lib, "default_params", _lib.NcsbParams)
     monkeypatch.setattr(ncs, "_on_device", lambda device: contextlib.nullcontext())
